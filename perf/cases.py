@@ -110,10 +110,13 @@ def _draw(rng):
     return {"kind": kind, "b": rng.choice([1, 2]), "heads": rng.choice([5, 10, 20]), "lq": lq, "slots": slots, "lslot": lslot}
 
 
-def prepare(case, seed):
+def _normal(seed):
     g = torch.Generator(device="cuda").manual_seed(seed)
-    rn = lambda *shape, scale=1.0, dtype=torch.float16: (torch.randn(*shape, device="cuda", generator=g) * scale).to(dtype)
-    return {"case": case, **_PREPARE[case["kind"]](case, rn)}
+    return lambda *shape, scale=1.0, dtype=torch.float16: (torch.randn(*shape, device="cuda", generator=g) * scale).to(dtype)
+
+
+def prepare(case, seed):
+    return {"case": case, **_PREPARE[case["kind"]](case, _normal(seed))}
 
 
 def _prepare_image(c, rn):
@@ -132,12 +135,12 @@ def _prepare_linear(c, rn):
             "residual": rn(m, n) if c["residual"] else None}
 
 
-def _prepare_lowp_linear(c, rn):
+def _prepare_lowp_linear(c, rn, wrap=BasedXLLowPLinear):
     layer = torch.nn.Linear(c["k"], c["n"], bias=c["bias"], device="cuda", dtype=torch.float16).requires_grad_(False)
     layer.weight.copy_(rn(c["n"], c["k"], scale=c["k"] ** -0.5))
     if c["bias"]:
         layer.bias.copy_(rn(c["n"]))
-    return {"x": rn(c["m"], c["k"]), "layer": BasedXLLowPLinear(layer)}
+    return {"x": rn(c["m"], c["k"]), "layer": wrap(layer)}
 
 
 def _prepare_matmul(c, rn):
@@ -145,10 +148,10 @@ def _prepare_matmul(c, rn):
     return {"a": rn(c["m"], c["k"], dtype=dtype), "b": rn(c["k"], c["n"], dtype=dtype)}
 
 
-def _prepare_conv(c, rn):
+def _prepare_conv(c, rn, pack=ops.conv_weight_pack):
     b, ci, co, h, w = c["b"], c["cin"], c["cout"], c["h"], c["w"]
     halo = rn(2, b, 1, w, ci)  # the staging range of a neighbouring strip: [side, image, row, column, channel]
-    return {"x": rn(b, h, w, ci), "weight": ops.conv_weight_pack(rn(co, ci, 3, 3, scale=(9 * ci) ** -0.5)), "bias": rn(co),
+    return {"x": rn(b, h, w, ci), "weight": pack(rn(co, ci, 3, 3, scale=(9 * ci) ** -0.5)), "bias": rn(co),
             "top": halo[1] if c["top"] else None, "bot": halo[0] if c["bot"] else None,
             "time_bias": rn(b, co) if c["time_bias"] else None,
             "residual": rn(b, h // c["stride"], w // c["stride"], co) if c["residual"] else None}
@@ -203,6 +206,92 @@ def _run_norm(s, mode):
     y = ops.groupnorm_fused(s["x"], GROUPS, 1e-5, s["gamma"], s["beta"], s["peers"], s["own"], ops.MODE_STALE, silu=True,
                             fresh_out=s["moments"], halo_out=s["halo"])
     return {"y": y, "moments": s["moments"], "halo": s["halo"]}
+
+
+def exact(case, seed):
+    """``run``'s outputs for the same inputs in 64 bits; an image would take minutes."""
+    return _EXACT[case["kind"]](case, _normal(seed)) if case["kind"] in _EXACT else None
+
+
+def _wide(state):
+    return {k: v.double() if isinstance(v, torch.Tensor) else v for k, v in state.items()}
+
+
+def _exact_linear(c, rn):
+    s = _wide(_prepare_linear(c, rn))
+    y = s["x"] @ s["weight"].T
+    if c["bias"]:
+        y += s["bias"]
+    return y + s["residual"] if c["residual"] else y
+
+
+def _exact_lowp_linear(c, rn):
+    s = _prepare_lowp_linear(c, rn, wrap=lambda layer: layer)
+    y = s["x"].double() @ s["layer"].weight.double().T
+    return y + s["layer"].bias.double() if c["bias"] else y
+
+
+def _exact_matmul(c, rn):
+    s = _wide(_prepare_matmul(c, rn))
+    return s["a"] @ s["b"]
+
+
+def _exact_conv(c, rn):
+    s = _wide(_prepare_conv(c, rn, pack=lambda w: w))
+    b, h, w, st = c["b"], c["h"], c["w"], c["stride"]
+    x = torch.zeros(b, h + 2, w + 2, c["cin"], device="cuda", dtype=torch.float64)
+    x[:, 1:-1, 1:-1] = s["x"]
+    if c["top"]:
+        x[:, :1, 1:-1] = s["top"]
+    if c["bot"]:
+        x[:, -1:, 1:-1] = s["bot"]
+    y = torch.zeros(b, h // st, w // st, c["cout"], device="cuda", dtype=torch.float64) + s["bias"]
+    for ky in range(3):
+        for kx in range(3):
+            y += x[:, ky : ky + h : st, kx : kx + w : st] @ s["weight"][:, :, ky, kx].T
+    if c["time_bias"]:
+        y += s["time_bias"][:, None, None, :]
+    return y + s["residual"] if c["residual"] else y
+
+
+def _exact_norm(c, rn):
+    raw = _prepare_norm(c, rn)
+    peers = torch.stack(raw["peers"]).double()
+    s = _wide(raw)
+    b, ch, h, w, own = c["b"], c["c"], c["h"], c["w"], s["own"]
+    x = s["x"].view(b, h * w, GROUPS, ch // GROUPS)
+    fresh = torch.stack([x.mean(dim=(1, 3)), (x * x).mean(dim=(1, 3))])
+    full = fresh
+    if c["mode"] == "stale":
+        full = peers.mean(dim=0) + fresh - peers[own]
+    elif c["mode"] == "sync":
+        peers[own] = fresh
+        full = peers.mean(dim=0)
+    var = full[1] - full[0] ** 2
+    var = torch.where(var < 0, fresh[1] - fresh[0] ** 2, var)
+    n = h * w * ch // GROUPS
+    rstd = (var * n / (n - 1) + 1e-5).rsqrt()
+    y = ((x - full[0][:, None, :, None]) * rstd[:, None, :, None]).reshape(b, h, w, ch)
+    y = torch.nn.functional.silu(y * s["gamma"] + s["beta"])
+    return y if c["mode"] == "local" else {"y": y, "moments": fresh, "halo": torch.stack([y[:, :1], y[:, -1:]])}
+
+
+def _exact_attention(c, rn):
+    s = _prepare_attention(c, rn)
+    b, lq, heads = c["b"], c["lq"], c["heads"]
+    split = lambda t: t.double().unflatten(-1, (heads, HEAD_DIM)).transpose(1, 2)
+    k, v = (split(t) for t in torch.cat(s["slots"], dim=1).chunk(2, dim=-1))
+    q = split(s["q"])
+    out = torch.empty(b, heads, lq, HEAD_DIM, device="cuda", dtype=torch.float64)
+    for i in range(0, lq, 1024):  # scores of 1024 queries at a time
+        for j in range(b):
+            p = (q[j, :, i : i + 1024] @ k[j].transpose(1, 2) * HEAD_DIM**-0.5).softmax(dim=-1)
+            out[j, :, i : i + 1024] = p @ v[j]
+    return out.transpose(1, 2).reshape(b, lq, heads * HEAD_DIM)
+
+
+_EXACT = {"linear": _exact_linear, "lowp_linear": _exact_lowp_linear, "matmul": _exact_matmul, "conv": _exact_conv,
+          "norm": _exact_norm, "attention": _exact_attention}
 
 
 def work(case):
