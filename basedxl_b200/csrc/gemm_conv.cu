@@ -54,19 +54,18 @@ constexpr int kEpiSub = BXL_EPI_SUB;            // epilogue warps per 32-row qua
 constexpr int kEpiThreads = kEpiSub * 128;
 constexpr int kWarpA = 4 * kEpiSub, kWarpMma = kWarpA + 1, kWarpB = kWarpA + 2;   // after the epilogue warps: A loads, MMA, B loads
 constexpr int kGemmThreads = (4 * kEpiSub + 3) * 32;
-constexpr int kMaxSeg = 3;
 constexpr int kABytes = kBM * kBK * 2;       // 16 KB
 constexpr int kSmemBudget = 227 * 1024;      // dynamic shared memory available to one CTA
 constexpr int kSmemMisc = 3072;              // alignment slack + barriers + the tile's bias row (256 floats)
 constexpr int kMaxStages = 8;
 
 struct alignas(64) GemmParams {
-  CUtensorMap a_map[kMaxSeg];  // GEMM: A of each segment.  conv: body (one row per copy), top halo, bottom halo
-  CUtensorMap b_map[kMaxSeg];  // GEMM: B of each segment.  conv: [0] = packed weights
+  CUtensorMap a_map[3];        // GEMM: A (split-operand product: hi, lo).  conv: body (one row per copy), top halo, bottom halo
+  CUtensorMap b_map[2];        // GEMM: B (split-operand product: hi, lo).  conv: [0] = packed weights
   CUtensorMap a_rows_map;      // conv: body again, with a box of `th` rows (one copy per stage)
   // problem
   int M, N, K;                 // conv: M = B*H_out*W_out (unused), N = C_out, K = 9*C_in
-  int nseg;                    // GEMM segments (1, or 3 for the split-operand product)
+  int parts;                   // fp16 parts of each operand (1, or 2 = hi and lo for the split-operand product)
   int b_kn;                    // B given as [K,N] row-major (MN-major operand) instead of [N,K]
   // tiling chosen by the host
   int bn;                      // tile width: multiple of 32, 32..256
@@ -261,7 +260,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
   const int BN = p.bn;
   const int S = kSplit ? p.split : 1;
   const int b_rows = kPair ? BN / 2 : BN;       // rows of the B tile this CTA stages
-  const int stage_bytes = kABytes + b_rows * 128;
+  const int parts = kConv ? 1 : p.parts;
+  const int b_bytes = b_rows * 128;
+  const int stage_bytes = parts * (kABytes + b_bytes);   // every part of A, then every part of B
   constexpr int kWidth = kPair ? 2 : 1;          // CTAs that cooperate on one tile (besides a K split)
   const uint32_t recv_base = smem_base + p.stages * stage_bytes;            // 1024-aligned (stage_bytes % 1024 == 0)
   const uint32_t bar_base = recv_base + recv_bytes(BN, S);
@@ -326,8 +327,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
   else tiles_m1 = (p.M + kBM - 1) / kBM;
   const int tiles_m = kPair ? (tiles_m1 + 1) / 2 : tiles_m1;  // scheduling units along M (pairs of tiles in pair mode)
   const int num_tiles = tiles_m * tiles_n;
-  const int kb_per_seg = kConv ? 9 * (p.cCin / kBK) : (p.K + kBK - 1) / kBK;
-  const int num_kb = kConv ? kb_per_seg : kb_per_seg * p.nseg;
+  const int num_kb = kConv ? 9 * (p.cCin / kBK) : (p.K + kBK - 1) / kBK;
   // this CTA's share of the K loop (balanced; never empty because split <= num_kb)
   const uint32_t krank = kPair ? 0u : crank;  // both CTAs of a pair walk the whole K range
   const int kb_begin = static_cast<int>((static_cast<long long>(krank) * num_kb) / S);
@@ -344,8 +344,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
     // (2048 x 5120 x 1280: 31.6 -> 26.4 us; stride-2 conv 2 x 640 x 64 x 64: 39.2 -> 31.5 us).
     const bool loads_a = (warp == kWarpA);
     if (elect_one()) {
-      for (int s = 0; s < kMaxSeg; ++s) tma_prefetch_desc(loads_a ? &p.a_map[s] : &p.b_map[s]);
-      if (loads_a && kConv) tma_prefetch_desc(&p.a_rows_map);
+      for (int s = 0; s < parts; ++s) tma_prefetch_desc(loads_a ? &p.a_map[s] : &p.b_map[s]);
+      if (loads_a && kConv) {
+        tma_prefetch_desc(&p.a_map[1]);
+        tma_prefetch_desc(&p.a_map[2]);
+        tma_prefetch_desc(&p.a_rows_map);
+      }
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -366,8 +370,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
         // position in the K loop, advanced without divisions: this thread's issue rate bounds the
         // pipeline ramp of short K loops
         const int cchunks = kConv ? p.cCin / kBK : 1;
-        int seg = kConv ? 0 : kb_begin / kb_per_seg;        // GEMM: operand segment and k-block inside it
-        int kk = kConv ? 0 : kb_begin % kb_per_seg;
         int tap = kConv ? kb_begin / cchunks : 0;           // conv: filter tap (ky, kx) and channel chunk
         int cc = kConv ? kb_begin % cchunks : 0;
         int ky = tap / 3, kx = tap % 3;
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
             break;
           }
           const uint32_t a_dst = smem_base + stage * stage_bytes;
-          const uint32_t b_dst = a_dst + kABytes;
+          const uint32_t b_dst = a_dst + parts * kABytes;
           // pair mode: both CTAs report their bytes to the leader's barrier; the leader's two
           // producer threads announce the bytes of both halves
           const uint32_t fbar = kPair ? map_to_cta(full_bar(stage), 0) : full_bar(stage);
@@ -391,7 +393,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
             else tma_load_5d(dst, m, fbar, c0, c1, c2, c3, c4);
           };
           if (loads_a) {
-            if (announces) mbar_arrive_expect_tx(full_bar(stage), kABytes * kWidth);
+            if (announces) mbar_arrive_expect_tx(full_bar(stage), parts * kABytes * kWidth);
             if (kConv) {
               const int c0 = cc * kBK;
               // input column of output column ox: stride*ox + kx - 1, addressed as
@@ -418,19 +420,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
                 }
               }
             } else {
-              load_2d(a_dst, &p.a_map[seg], kk * kBK, tm * kBM);
+              load_2d(a_dst, &p.a_map[0], kb * kBK, tm * kBM);
+              if (parts == 2) load_2d(a_dst + kABytes, &p.a_map[1], kb * kBK, tm * kBM);
             }
           } else {
-            if (announces) mbar_arrive_expect_tx(full_bar(stage), b_rows * 128 * kWidth);
+            if (announces) mbar_arrive_expect_tx(full_bar(stage), parts * b_bytes * kWidth);
             if (kConv) {
               load_2d(b_dst, &p.b_map[0], kb * kBK, n0);
             } else {
-              const int k0 = kk * kBK;
+              const int k0 = kb * kBK;
               if (p.b_kn) {
                 // B[K,N]: one 64(n) x 64(k) box per 64 output columns
-                for (int j = 0; j < b_rows / 64; ++j) load_2d(b_dst + j * 8192, &p.b_map[seg], n0 + j * 64, k0);
+                for (int s = 0; s < parts; ++s)
+                  for (int j = 0; j < b_rows / 64; ++j) load_2d(b_dst + s * b_bytes + j * 8192, &p.b_map[s], n0 + j * 64, k0);
               } else {
-                load_2d(b_dst, &p.b_map[seg], k0, n0);
+                load_2d(b_dst, &p.b_map[0], k0, n0);
               }
             }
           }
@@ -443,8 +447,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
               cc = 0;
               if (++kx == 3) kx = 0, ++ky;
             }
-          } else if (++kk == kb_per_seg) {
-            kk = 0, ++seg;
           }
         }
       }
@@ -475,16 +477,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
           }
           tc_fence_after_sync();
           const uint32_t a_addr = smem_base + stage * stage_bytes;
-          const uint32_t b_addr = a_addr + kABytes;
+          const uint32_t b_addr = a_addr + parts * kABytes;
           const uint64_t adesc = make_smem_desc_sw128(a_addr, 16, 1024);
           const uint32_t first = (kb == kb_begin) ? 0u : 1u;
           if (!kConv && p.b_kn) {
             // MN-major B: 64-column chunks 8 KB apart (LBO), 8-row k-groups 1 KB apart (SBO)
             const uint64_t bdesc = make_smem_desc_sw128(b_addr, 8192, 1024);
+            // split operands: hi*hi, hi*lo, lo*hi into the same accumulator, each part staged once
+            for (int t = 0; t < 2 * parts - 1; ++t) {
+              const uint64_t ad = adesc + (t == 2 ? kABytes / 16 : 0);
+              const uint64_t bd = bdesc + (t == 1 ? b_bytes / 16 : 0);
 #pragma unroll
-            for (int k = 0; k < kBK / kUmmaK; ++k) {
-              if (kPair) umma_f16_pair(d_tmem, adesc + 2u * k, bdesc + 128u * k, idesc, first | k);
-              else umma_f16(d_tmem, adesc + 2u * k, bdesc + 128u * k, idesc, first | k);
+              for (int k = 0; k < kBK / kUmmaK; ++k) {
+                if (kPair) umma_f16_pair(d_tmem, ad + 2u * k, bd + 128u * k, idesc, first | k | t);
+                else umma_f16(d_tmem, ad + 2u * k, bd + 128u * k, idesc, first | k | t);
+              }
             }
           } else {
             const uint64_t bdesc = make_smem_desc_sw128(b_addr, 16, 1024);
@@ -717,8 +724,8 @@ struct TileConfig {
 
 constexpr int kSmemLnExtra = 1024;           // the weight column-sum row of a GEMM with a folded LayerNorm
 
-static int stages_for(int bn, int split, int pair = 0, int extra_smem = 0) {
-  const int stage = kABytes + (pair ? bn * 64 : bn * 128);
+static int stages_for(int bn, int split, int pair = 0, int extra_smem = 0, int parts = 1) {
+  const int stage = parts * (kABytes + (pair ? bn * 64 : bn * 128));
   int st = (kSmemBudget - kSmemMisc - extra_smem - recv_bytes(bn, split)) / stage;
   if (st > kMaxStages) st = kMaxStages;
   return st;
@@ -734,9 +741,9 @@ static int stages_for(int bn, int split, int pair = 0, int extra_smem = 0) {
 // convolution).  A wider tile or a pair moves fewer bytes per FLOP; a narrower tile or a K split
 // spreads the stream over more SMs when there are few tiles.
 static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int force_bn = 0, int force_split = 0,
-                               int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0) {
+                               int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0, int parts = 1) {
   const int sms = sm_count();
-  TileConfig best{128, 1, stages_for(128, 1, 0, extra_smem), 0};
+  TileConfig best{128, 1, stages_for(128, 1, 0, extra_smem, parts), 0};
   double best_cost = 1e30;
   for (int pair = 0; pair <= 1; ++pair) {
     if (force_pair >= 0 && pair != force_pair) continue;
@@ -748,14 +755,14 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
       for (int split = 1; split <= (pair ? 1 : 4); split *= 2) {
         if (force_split && split != force_split) continue;
         if ((bn / 32) % split || split > num_kb) continue;
-        const int st = stages_for(bn, split, pair, extra_smem);
+        const int st = stages_for(bn, split, pair, extra_smem, parts);
         if (st < 3) continue;
         const int width = pair ? 2 : split;
         const int clusters = sms / width;
         const int par = tiles < clusters ? tiles : clusters;
         const int rounds = (tiles + par - 1) / par;
         const double bytes = 16384.0 + bn * (pair ? 64.0 : 128.0);
-        const double kb_us = fmax(fmax(bn / 256.0 * 0.27, pair ? 0.24 + 0.00063 * bn : bytes / 110000.0), a_min_us);
+        const double kb_us = fmax(fmax((2 * parts - 1) * bn / 256.0 * 0.27, parts * (pair ? 0.24 + 0.00063 * bn : bytes / 110000.0)), a_min_us);
         const double kb_unit = (num_kb + split - 1) / split;
         const double epi_us = 0.08 * (bn / 32.0) / split + (split > 1 ? 1.2 : 0.0);  // accumulator read-out (+ exchange)
         const double fill_us = 1.0 + (st < 4 ? 0.5 : 0.0) + (pair ? 0.3 : 0.0);       // pipeline ramp per unit
@@ -774,7 +781,7 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
 template <bool kConv, bool kPair, bool kSplit>
 static int launch_one(const GemmParams& p, int num_units, cudaStream_t stream) {
   const int b_rows = kPair ? p.bn / 2 : p.bn;
-  const int smem = p.stages * (kABytes + b_rows * 128) + recv_bytes(p.bn, kSplit ? p.split : 1) + kSmemMisc +
+  const int smem = p.stages * p.parts * (kABytes + b_rows * 128) + recv_bytes(p.bn, kSplit ? p.split : 1) + kSmemMisc +
                    (p.ln_part ? kSmemLnExtra : 0);
   static bool configured[64] = {};
   int dev = 0;
@@ -854,11 +861,7 @@ extern "C" int bxl_gemm_f16(const void* A, long long lda, const void* B, long lo
     uint32_t box[2] = {kBK, (uint32_t)(tc.pair ? BN / 2 : BN)};
     if (int rc = encode_tmap_f16(&p.b_map[0], B, 2, dims, str, box)) return rc;
   }
-  for (int s = 1; s < kMaxSeg; ++s) {
-    p.a_map[s] = p.a_map[0];
-    p.b_map[s] = p.b_map[0];
-  }
-  p.M = M, p.N = N, p.K = K, p.nseg = 1, p.b_kn = b_is_kn ? 1 : 0;
+  p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = b_is_kn ? 1 : 0;
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
@@ -895,11 +898,7 @@ extern "C" int bxl_gemm_dual_f16(const void* A, long long lda, const void* B, lo
     uint32_t box[2] = {kBK, (uint32_t)(tc.pair ? tc.bn / 2 : tc.bn)};
     if (int rc = encode_tmap_f16(&p.b_map[0], B, 2, dims, str, box)) return rc;
   }
-  for (int s = 1; s < kMaxSeg; ++s) {
-    p.a_map[s] = p.a_map[0];
-    p.b_map[s] = p.b_map[0];
-  }
-  p.M = M, p.N = N, p.K = K, p.nseg = 1, p.b_kn = 0;
+  p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 0;
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
@@ -933,11 +932,7 @@ extern "C" int bxl_gemm_geglu_f16(const void* A, long long lda, const void* B, l
     uint32_t box[2] = {kBK, (uint32_t)(tc.pair ? tc.bn / 2 : tc.bn)};
     if (int rc = encode_tmap_f16(&p.b_map[0], B, 2, dims, str, box)) return rc;
   }
-  for (int s = 1; s < kMaxSeg; ++s) {
-    p.a_map[s] = p.a_map[0];
-    p.b_map[s] = p.b_map[0];
-  }
-  p.M = M, p.N = N, p.K = K, p.nseg = 1, p.b_kn = 0;
+  p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 0;
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
@@ -1000,11 +995,7 @@ extern "C" int bxl_gemm_fused_f16(const bxl_gemm_fused_args* a, int* row_stats_p
     uint32_t box[2] = {kBK, (uint32_t)(tc.pair ? tc.bn / 2 : tc.bn)};
     if (int rc = encode_tmap_f16(&p.b_map[0], a->B, 2, dims, str, box)) return rc;
   }
-  for (int s = 1; s < kMaxSeg; ++s) {
-    p.a_map[s] = p.a_map[0];
-    p.b_map[s] = p.b_map[0];
-  }
-  p.M = M, p.N = N, p.K = K, p.nseg = 1, p.b_kn = 0;
+  p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 0;
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(a->bias);
@@ -1038,17 +1029,30 @@ extern "C" int bxl_debug_force_tile_order(int order) {
 // ---- split-operand product of fp32 matrices ---------------------------------------
 namespace bxl {
 // x = hi + lo with hi = fp16(x), lo = fp16(x - hi): 22 significant bits kept.
-__global__ void split_f32_kernel(const float* __restrict__ x, __half* __restrict__ hi, __half* __restrict__ lo, long long n4) {
+// Both operands in one launch (their parts lie back to back: a_hi, a_lo, b_hi, b_lo); eight values per
+// thread and step, so that every load and store is a whole 16-byte vector.  Bound by memory.
+__global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict__ a, const float* __restrict__ b,
+                                                        __half* __restrict__ parts, long long na, long long nb) {
   pdl_launch_dependents();
   pdl_wait();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
-    const float4 v = reinterpret_cast<const float4*>(x)[i];
-    const __half h0 = __float2half_rn(v.x), h1 = __float2half_rn(v.y), h2 = __float2half_rn(v.z), h3 = __float2half_rn(v.w);
-    __half2 hh[2] = {__halves2half2(h0, h1), __halves2half2(h2, h3)};
-    __half2 ll[2] = {__floats2half2_rn(v.x - __half2float(h0), v.y - __half2float(h1)),
-                     __floats2half2_rn(v.z - __half2float(h2), v.w - __half2float(h3))};
-    reinterpret_cast<uint2*>(hi)[i] = *reinterpret_cast<uint2*>(hh);
-    reinterpret_cast<uint2*>(lo)[i] = *reinterpret_cast<uint2*>(ll);
+  const long long na8 = na / 8, n8 = na8 + nb / 8;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+    const bool of_a = i < na8;
+    const long long e = 8 * (of_a ? i : i - na8);
+    const float* x = (of_a ? a : b) + e;
+    __half* hi = parts + (of_a ? 0 : 2 * na) + e;
+    __half* lo = hi + (of_a ? na : nb);
+    const float4 v[2] = {__ldcs(reinterpret_cast<const float4*>(x)), __ldcs(reinterpret_cast<const float4*>(x) + 1)};
+    __half2 hh[4], ll[4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const __half h0 = __float2half_rn(v[j].x), h1 = __float2half_rn(v[j].y), h2 = __float2half_rn(v[j].z), h3 = __float2half_rn(v[j].w);
+      hh[2 * j] = __halves2half2(h0, h1), hh[2 * j + 1] = __halves2half2(h2, h3);
+      ll[2 * j] = __floats2half2_rn(v[j].x - __half2float(h0), v[j].y - __half2float(h1));
+      ll[2 * j + 1] = __floats2half2_rn(v[j].z - __half2float(h2), v[j].w - __half2float(h3));
+    }
+    *reinterpret_cast<uint4*>(hi) = *reinterpret_cast<uint4*>(hh);
+    *reinterpret_cast<uint4*>(lo) = *reinterpret_cast<uint4*>(ll);
   }
 }
 }  // namespace bxl
@@ -1074,19 +1078,23 @@ extern "C" int bxl_gemm_split_f32(const float* A, const float* B, float* C, int 
   __half* a_lo = a_hi + na;
   __half* b_hi = a_lo + na;
   __half* b_lo = b_hi + nb;
-  const int blocks = sm_count() * 8;
-  split_f32_kernel<<<blocks, 256, 0, s>>>(A, a_hi, a_lo, na / 4);
-  split_f32_kernel<<<blocks, 256, 0, s>>>(B, b_hi, b_lo, nb / 4);
-  if (int rc = check_cuda(cudaGetLastError(), "split_f32_kernel launch")) return rc;
+  const long long blocks = ((na + nb) / 8 + 255) / 256, most = sm_count() * 8;
+  if (int rc = launch_kernel("split_f32_kernel launch", split_f32_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s,
+                             1, A, B, a_hi, na, nb))
+    return rc;
   GemmParams p;
   memset(&p, 0, sizeof(p));
   const int tiles_m = (M + kBM - 1) / kBM;
-  const TileConfig tc = choose_tiles(tiles_m, N, 3 * ((K + kBK - 1) / kBK), true, g_force_bn, g_force_split, g_force_pair < 0 ? kDefaultPair : g_force_pair);
+  const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, true, g_force_bn, g_force_split,
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, 0, 2);
   const int BN = tc.bn;
-  // C = A_hi*B_hi + A_hi*B_lo + A_lo*B_hi, one fp32 accumulator
-  const __half* as[3] = {a_hi, a_hi, a_lo};
-  const __half* bs[3] = {b_hi, b_lo, b_hi};
-  for (int i = 0; i < 3; ++i) {
+  // C = A_hi*B_hi + A_hi*B_lo + A_lo*B_hi, one fp32 accumulator.  The operand stream bounds the K loop, so a
+  // ring slot holds the four parts of a k-block and three products are formed from it (four tiles copied for
+  // three products; one product at a time copied six): 8192 x 640 x 640 42.3 -> 33.8 us, 4096 x 2048 x 2048
+  // 98.4 -> 86.6 us, 256 x 512 x 512 14.5 -> 9.4 us, the parts in one launch included.
+  const __half* as[2] = {a_hi, a_lo};
+  const __half* bs[2] = {b_hi, b_lo};
+  for (int i = 0; i < 2; ++i) {
     uint64_t ad[2] = {(uint64_t)K, (uint64_t)M};
     uint64_t astr[1] = {(uint64_t)K * 2};
     uint32_t abox[2] = {kBK, kBM};
@@ -1096,7 +1104,7 @@ extern "C" int bxl_gemm_split_f32(const float* A, const float* B, float* C, int 
     uint32_t bbox[2] = {64, kBK};
     if (int rc = encode_tmap_f16(&p.b_map[i], bs[i], 2, bd, bstr, bbox)) return rc;
   }
-  p.M = M, p.N = N, p.K = K, p.nseg = 3, p.b_kn = 1;
+  p.M = M, p.N = N, p.K = K, p.parts = 2, p.b_kn = 1;
   // b_static stays 0: the fp16 parts of B were written by the kernel launched just above
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair;
   p.C = C, p.ldc = N, p.out_f32 = 1;
@@ -1181,9 +1189,7 @@ extern "C" int bxl_conv3x3_halo_f16(const void* x, long long x_img_stride, const
     uint32_t box[2] = {kBK, (uint32_t)(tc.pair ? BN / 2 : BN)};
     if (int rc = encode_tmap_f16(&p.b_map[0], w_packed, 2, dims, str, box)) return rc;
   }
-  p.b_map[1] = p.b_map[0];
-  p.b_map[2] = p.b_map[0];
-  p.M = B * H_out * W_out, p.N = C_out, p.K = K, p.nseg = 1, p.b_kn = 0;
+  p.M = B * H_out * W_out, p.N = C_out, p.K = K, p.parts = 1, p.b_kn = 0;
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
   p.bias = static_cast<const __half*>(bias);
   p.bias_rows = static_cast<const __half*>(bias_rows);

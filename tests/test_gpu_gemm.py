@@ -352,3 +352,24 @@ def test_layernorm_folded_into_gemm(kind, bn, split, pair):
     finally:
         _lib.check(l.bxl_debug_force_tiles(0, 0, -1), l, kernels=0)
     assert_close(y, ref, what=f"LayerNorm folded into {kind} GEMM (bn={bn} split={split} pair={pair})")
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 8, 8), (127, 64, 72), (129, 72, 128), (300, 200, 136), (256, 1280, 384), (2048, 640, 1288)])
+@pytest.mark.parametrize("split,pair", [(0, -1), (2, 0), (1, 1)])
+def test_split_product_edges(M, K, N, split, pair):
+    """fp32 operands with both fp16 parts staged in one ring slot: K tails, ragged tiles, K splits and CTA pairs.
+    Bound: the dropped lo*lo term and the parts' rounding (2^-22 of each product) plus the truncating fp32
+    accumulation (at most 2^-23 of the running sum per 16-deep step, three products each)."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    g = torch.Generator().manual_seed(M + K + N)
+    a, b = torch.randn(M, K, generator=g), torch.randn(K, N, generator=g)
+    l = _lib.lib()
+    _lib.check(l.bxl_debug_force_tiles(0, split, pair), l, kernels=0)
+    try:
+        y = ops.gemm_split_f32(a.to(dev), b.to(dev)).cpu().double()
+        _lib.device_status()
+    finally:
+        _lib.check(l.bxl_debug_force_tiles(0, 0, -1), l, kernels=0)
+    bound = (2.0**-21 + 3 * (K / 16 + 1) * 2.0**-23) * (a.abs().double() @ b.abs().double())
+    assert bool(((y - a.double() @ b.double()).abs() <= bound).all())
