@@ -56,20 +56,19 @@ def cascaded_lowp_matmul(
             return out
         return res.reshape(*batch_dims, N)
     if K % 8 or N % 8:
-        # rows must be whole 16-byte vectors for the copy engine: zero-pad K and N
-        Kp, Np = (K + 7) // 8 * 8, (N + 7) // 8 * 8
-        a_p = torch.zeros(a2.shape[0], Kp, device=a.device, dtype=a.dtype)
-        a_p[:, :K] = a2
-        b_p = torch.zeros(Kp, Np, device=b.device, dtype=b.dtype)
-        b_p[:K, :N] = b
-        res = ops.gemm(a_p, b_p, b_is_kn=True)[:, :N]
-        if bias is not None:
+        # the kernel adds a plain fp16 row of N values; any other bias is added to the product
+        fused = bias if bias is not None and bias.is_cuda and bias.dtype == torch.float16 and bias.shape == (N,) and bias.stride(0) == 1 else None
+        r2 = None if residual is None else residual.reshape(-1, N)
+        if r2 is not None and r2.stride(1) != 1:
+            r2 = r2.contiguous()
+        res = ops.gemm_ragged(a2, b, bias=fused, residual=r2)
+        if bias is not None and fused is None:
             res = res + bias
         res = res.reshape(*batch_dims, N)
         if out is not None:
             out.copy_(res)
             return out
-        return res.contiguous()
+        return res
     o2 = None if out is None else out.view(-1, N)
     r2 = None if residual is None else residual.reshape(-1, N)
     res = ops.gemm(a2, b, bias=bias, residual=r2, out=o2, b_is_kn=True)

@@ -102,6 +102,7 @@ struct alignas(64) GemmParams {
   // (sum, sum of squares) per row and per column slice a CTA owns, [M][stat_parts].
   float2* stat_out;
   int stat_parts;
+  int ragged;                  // rows of C (and of the residual) are not 16-byte aligned: chunks go through a transposing stage
   // conv geometry
   int cB, cHin, cW, cCin, cStride, cHout, cWout;
   int tw, th;                  // tile = th rows x tw columns of output pixels (th*tw = 128)
@@ -124,7 +125,7 @@ struct ResidualChunk {
   bool valid;
 };
 __device__ __forceinline__ void load_residual(const GemmParams& p, long long out_row, int nb, ResidualChunk& r) {
-  r.valid = (p.residual != nullptr) && out_row >= 0 && (nb + 32 <= p.N);
+  r.valid = (p.residual != nullptr) && !p.ragged && out_row >= 0 && (nb + 32 <= p.N);
   if (r.valid) {
     const __half* rr = p.residual + out_row * p.ldr + nb;
 #pragma unroll
@@ -249,6 +250,29 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, float (&f)[32],
   }
 }
 
+// Rows of C whose stride is no multiple of 16 bytes cannot take a thread's 64 bytes as vectors, and one
+// element per lane and row would touch 32 sectors per store.  The warp turns the chunk in shared memory
+// ([32 rows][33 floats], conflict-free both ways) and stores row by row: 32 neighbouring elements at a time.
+// All 32 lanes call it; `row0` is the first of the warp's 32 output rows.
+constexpr int kTurnFloats = 32 * 33;
+__device__ __forceinline__ void store_chunk_ragged(const GemmParams& p, const float (&f)[32], int row0, int nb, const float* sbias,
+                                                   float* turn, int lane) {
+  __syncwarp();   // the previous chunk has been stored
+#pragma unroll
+  for (int j = 0; j < 32; ++j) turn[lane * 33 + j] = f[j];
+  __syncwarp();
+  const int col = nb + lane;
+  if (col >= p.N) return;
+  const float b = sbias ? sbias[lane] : 0.f;
+  const int rows = min(32, p.M - row0);
+  for (int r = 0; r < rows; ++r) {
+    float v = turn[r * 33 + lane] + b;
+    const long long m = row0 + r;
+    if (p.residual) v += __half2float(p.residual[m * p.ldr + col]);
+    static_cast<__half*>(p.C)[m * p.ldc + col] = __float2half_rn(v);
+  }
+}
+
 // kSplit: the K loop is split over the CTAs of a cluster (p.split of them); a separate
 // instantiation, so that each variant carries only its own epilogue (and its registers).
 template <bool kConv, bool kPair, bool kSplit>
@@ -278,6 +302,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 8);
   float* s_bias = reinterpret_cast<float*>(misc + 256);   // [256]: bias row of the tile in the epilogue
   float* s_colsum = s_bias + 256;                         // [256]: weight column sums (LayerNorm fold only; the host sizes the CTA for it)
+
+  float* s_turn = s_colsum;                               // [epilogue warps][kTurnFloats]: only with ragged rows (never beside the LayerNorm fold)
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5;
@@ -609,7 +635,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
           if (c + kEpiSub < chunks) load_residual(p, out_row, n0 + (c + kEpiSub) * 32, res_next);
           tmem_ld_wait();
           const int nb = n0 + c * 32;
-          if (out_row >= 0 && nb < p.N) {
+          if (!kConv && p.ragged) {
+            float f[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+            store_chunk_ragged(p, f, tm * kBM + quarter * 32, nb, has_bias ? s_bias + c * 32 : nullptr, s_turn + warp * kTurnFloats, lane);
+          } else if (out_row >= 0 && nb < p.N) {
             float f[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
@@ -674,7 +705,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
             }
           }
           const int nb = n0 + c * 32;
-          if (out_row >= 0 && nb < p.N)
+          if (!kConv && p.ragged)
+            store_chunk_ragged(p, f, tm * kBM + quarter * 32, nb, has_bias ? s_bias + c * 32 : nullptr, s_turn + warp * kTurnFloats, lane);
+          else if (out_row >= 0 && nb < p.N)
             store_chunk<kConv>(p, f, out_row, nb, img, has_bias ? s_bias + c * 32 : nullptr, res_cur,
                                has_ln ? s_colsum + c * 32 : nullptr, ln, stat);
           res_cur = res_next;
@@ -723,6 +756,7 @@ struct TileConfig {
 };
 
 constexpr int kSmemLnExtra = 1024;           // the weight column-sum row of a GEMM with a folded LayerNorm
+constexpr int kSmemRaggedExtra = 4 * kEpiSub * kTurnFloats * 4;   // the epilogue warps' transposing stages
 
 static int stages_for(int bn, int split, int pair = 0, int extra_smem = 0, int parts = 1) {
   const int stage = parts * (kABytes + (pair ? bn * 64 : bn * 128));
@@ -782,7 +816,7 @@ template <bool kConv, bool kPair, bool kSplit>
 static int launch_one(const GemmParams& p, int num_units, cudaStream_t stream) {
   const int b_rows = kPair ? p.bn / 2 : p.bn;
   const int smem = p.stages * p.parts * (kABytes + b_rows * 128) + recv_bytes(p.bn, kSplit ? p.split : 1) + kSmemMisc +
-                   (p.ln_part ? kSmemLnExtra : 0);
+                   (p.ln_part ? kSmemLnExtra : 0) + (p.ragged ? kSmemRaggedExtra : 0);
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -869,6 +903,115 @@ extern "C" int bxl_gemm_f16(const void* A, long long lda, const void* B, long lo
   p.ldr = ldr, p.C = C, p.ldc = ldc, p.out_f32 = out_f32 ? 1 : 0;
   p.dev_status = st;
   return launch<false>(p, tiles_m, (N + BN - 1) / BN, (cudaStream_t)stream);
+}
+
+// ---- product of matrices whose rows are not 16-byte aligned -------------------------
+namespace bxl {
+// Copies an operand's rows to 16-byte aligned ones (the copy engine reads nothing else), both operands in one
+// launch.  Bound by memory: a thread reads its eight values as four 32-bit words (three, and two single values,
+// where they start at an odd one), shifts them into place and stores one 16-byte vector.  Columns past the row's
+// end are not written: the tensor map ends at the row's end.
+struct RepackOperand {
+  const __half* src;
+  __half* dst;          // null: this operand is used where it is
+  long long ld, ld_dst; // elements
+  int rows, cols;
+};
+__device__ __forceinline__ void repack_vector(const RepackOperand& o, long long i) {
+  const int vecs = static_cast<int>(o.ld_dst / 8);
+  const long long r = i / vecs;
+  const int c = static_cast<int>(i % vecs) * 8;
+  const uint16_t* s = reinterpret_cast<const uint16_t*>(o.src + r * o.ld + c);
+  uint16_t* d = reinterpret_cast<uint16_t*>(o.dst + r * o.ld_dst + c);
+  const int n = min(8, o.cols - c);
+  if (n == 8) {
+    uint32_t w[4];
+    if ((reinterpret_cast<uintptr_t>(s) & 2u) == 0) {
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(s);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = __ldg(q + j);
+    } else {
+      const uint32_t* q = reinterpret_cast<const uint32_t*>(s + 1);
+      const uint32_t a = __ldg(s), b = __ldg(q), e = __ldg(q + 1), f = __ldg(q + 2), g = __ldg(s + 7);
+      w[0] = a | (b << 16), w[1] = __funnelshift_r(b, e, 16), w[2] = __funnelshift_r(e, f, 16), w[3] = (f >> 16) | (g << 16);
+    }
+    *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+    for (int j = 0; j < n; ++j) d[j] = s[j];
+  }
+}
+__global__ void __launch_bounds__(256) repack_rows_kernel(const RepackOperand a, const RepackOperand b) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long na = a.dst ? a.rows * (a.ld_dst / 8) : 0, n = na + (b.dst ? b.rows * (b.ld_dst / 8) : 0);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    if (i < na) repack_vector(a, i);
+    else repack_vector(b, i - na);
+  }
+}
+static bool rows_aligned(const void* base, long long ld, int cols) { return aligned16(base) && ld % 8 == 0 && ld >= cols; }
+static long long round8(long long n) { return (n + 7) / 8 * 8; }
+}  // namespace bxl
+
+extern "C" long long bxl_gemm_ragged_workspace_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  return 2ll * (M * round8(K) + K * round8(N));
+}
+
+extern "C" int bxl_gemm_ragged_f16(const void* A, long long lda, const void* B, long long ldb, const void* bias, const void* residual,
+                                   long long ldr, void* C, long long ldc, int M, int N, int K, void* workspace,
+                                   long long workspace_bytes, void* stream) {
+  if (!A || !B || !C || !workspace) return fail(kErrInvalidArg, "bxl_gemm_ragged_f16: null pointer");
+  if (M <= 0 || N <= 0 || K <= 0) return fail(kErrInvalidArg, "bxl_gemm_ragged_f16: non-positive extent M=%d N=%d K=%d", M, N, K);
+  if (lda < 0 || ldb < 0 || ldr < 0 || ldc < N) return fail(kErrInvalidArg, "bxl_gemm_ragged_f16: bad leading dimension");
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) |
+       reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(bias)) & 1u)
+    return fail(kErrInvalidArg, "bxl_gemm_ragged_f16: operands must be 2-byte aligned");
+  if (!aligned16(workspace)) return fail(kErrInvalidArg, "bxl_gemm_ragged_f16: workspace must be 16-byte aligned");
+  if (workspace_bytes < bxl_gemm_ragged_workspace_bytes(M, N, K)) return fail(kErrTooLarge, "bxl_gemm_ragged_f16: workspace too small");
+  int* st = device_status_ptr();
+  if (!st) return fail(kErrCuda, "bxl_gemm_ragged_f16: no device status word");
+  cudaStream_t s = (cudaStream_t)stream;
+  RepackOperand a{static_cast<const __half*>(A), nullptr, lda, lda, M, K}, b{static_cast<const __half*>(B), nullptr, ldb, ldb, K, N};
+  __half* ws = static_cast<__half*>(workspace);
+  if (!rows_aligned(A, lda, K)) a.dst = ws, a.ld_dst = round8(K);
+  if (!rows_aligned(B, ldb, N)) b.dst = ws + M * round8(K), b.ld_dst = round8(N);
+  const long long vecs = (a.dst ? M * (a.ld_dst / 8) : 0) + (b.dst ? K * (b.ld_dst / 8) : 0);
+  if (vecs > 0) {
+    const long long blocks = (vecs + 255) / 256, most = sm_count() * 8;
+    if (int rc = launch_kernel("repack_rows_kernel launch", repack_rows_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256),
+                               0, s, 1, a, b))
+      return rc;
+  }
+  GemmParams p;
+  memset(&p, 0, sizeof(p));
+  // Rows that happen to be aligned take the vector epilogue.  Copying both operands to padded buffers, a product
+  // with padded columns and a copy back took 68 us at 1000 x 1003 x 1501; this takes 27 us, most of it host time.
+  const bool ragged = !aligned16(C) || ldc % 8 || N % 8 || (residual && (!aligned16(residual) || ldr % 8));
+  const int tiles_m = (M + kBM - 1) / kBM;
+  const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, true, g_force_bn, g_force_split,
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, ragged ? kSmemRaggedExtra : 0);
+  {
+    uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
+    uint64_t str[1] = {(uint64_t)a.ld_dst * 2};
+    uint32_t box[2] = {kBK, kBM};
+    if (int rc = encode_tmap_f16(&p.a_map[0], a.dst ? a.dst : a.src, 2, dims, str, box)) return rc;
+  }
+  {
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)K};
+    uint64_t str[1] = {(uint64_t)b.ld_dst * 2};
+    uint32_t box[2] = {64, kBK};
+    if (int rc = encode_tmap_f16(&p.b_map[0], b.dst ? b.dst : b.src, 2, dims, str, box)) return rc;
+  }
+  p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 1;
+  // B is not static where the kernel above has just written it
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = (static_weights() && !b.dst) ? 1 : 0;
+  p.n_fastest = linear_tile_order(M, N, K, tc.bn);
+  p.bias = static_cast<const __half*>(bias);
+  p.residual = static_cast<const __half*>(residual);
+  p.ldr = ldr, p.C = C, p.ldc = ldc, p.ragged = ragged ? 1 : 0;
+  p.dev_status = st;
+  return launch<false>(p, tiles_m, (N + tc.bn - 1) / tc.bn, s);
 }
 
 extern "C" int bxl_gemm_dual_f16(const void* A, long long lda, const void* B, long long ldb, const void* bias, void* C1,

@@ -206,6 +206,27 @@ def gemm_fused(a, w, *, bias=None, bias_f32=None, residual=None, out=None, out2=
     return (out, stats) if want_stats else out
 
 
+def gemm_ragged(a, b, bias=None, residual=None):
+    """``a[M,K] @ b[K,N] (+ bias) (+ residual)`` for matrices whose rows are not 16-byte aligned.  ``b`` is
+    contiguous; the rows of ``a`` and ``residual`` are unit-stride, any distance apart."""
+    _f16_cuda(a, "a"), _f16_cuda(b, "b")
+    M, K = a.shape
+    N = b.shape[1]
+    _req(b.shape[0] == K, "gemm_ragged: inner dimensions differ")
+    if residual is not None:
+        _f16_cuda(residual, "residual")
+        _req(residual.shape == (M, N), "gemm_ragged: bad residual")
+    out = torch.empty((M, N), device=a.device, dtype=torch.float16)
+    l = _lib.lib()
+    ws = torch.empty(max(l.bxl_gemm_ragged_workspace_bytes(M, N, K), 16), device=a.device, dtype=torch.uint8)
+    _lib.check(
+        l.bxl_gemm_ragged_f16(_p(a), a.stride(0), _p(b), N, _p(bias), _p(residual), 0 if residual is None else residual.stride(0),
+                              _p(out), N, M, N, K, _p(ws), ws.numel(), _stream()),
+        l, kernels=2,
+    )
+    return out
+
+
 def gemm_split_f32(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """fp32 ``a[M,K] @ b[K,N]`` through the split-operand tensor-core product."""
     _req(a.is_cuda and a.dtype == torch.float32 and b.dtype == torch.float32, "gemm_split_f32: CUDA fp32 operands")

@@ -141,6 +141,15 @@ long long bxl_gemm_split_workspace_bytes(int M, int N, int K);
 int bxl_gemm_split_f32(const float* A, const float* B, float* C, int M, int N, int K, void* workspace,
                        long long workspace_bytes, void* stream);
 
+/* fp16 product of row-major matrices whose rows need not be 16-byte aligned: A[M,K] (rows lda elements
+ * apart, any distance), B[K,N] (ldb), C[M,N] (ldc >= N), all 2-byte aligned.  Operands that the copy engine
+ * cannot read are first copied to aligned rows in `workspace`.  Replaces: the same reference kernel as
+ * bxl_gemm_f16 (its masked loads and stores, basedxl/triton/cascaded_lowp_matmul.py:54-136). */
+long long bxl_gemm_ragged_workspace_bytes(int M, int N, int K);
+int bxl_gemm_ragged_f16(const void* A, long long lda, const void* B, long long ldb, const void* bias, const void* residual,
+                        long long ldr, void* C, long long ldc, int M, int N, int K, void* workspace, long long workspace_bytes,
+                        void* stream);
+
 /* ---- convolution ---------------------------------------------------------- */
 
 /* [C_out][C_in][3][3] -> [C_out][ky][kx][C_in], the weight layout both

@@ -373,3 +373,32 @@ def test_split_product_edges(M, K, N, split, pair):
         _lib.check(l.bxl_debug_force_tiles(0, 0, -1), l, kernels=0)
     bound = (2.0**-21 + 3 * (K / 16 + 1) * 2.0**-23) * (a.abs().double() @ b.abs().double())
     assert bool(((y - a.double() @ b.double()).abs() <= bound).all())
+
+
+@pytest.mark.parametrize(
+    "M,K,N",
+    [(1, 1, 1), (5, 7, 9), (31, 64, 33), (128, 65, 128), (127, 128, 127), (129, 1003, 257), (300, 200, 135), (1000, 1003, 1501), (2100, 333, 1001)],
+)
+@pytest.mark.parametrize("a_form", ["plain", "offset", "wide_rows", "one_row"])
+@pytest.mark.parametrize("epilogue", [False, True])
+def test_matmul_with_unaligned_rows(M, K, N, a_form, epilogue):
+    """Extents, row strides and addresses that are no multiple of 16 bytes, with and without bias and residual."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    from basedxl_b200.cascaded_lowp_matmul import cascaded_lowp_matmul
+
+    g = torch.Generator().manual_seed(M + 3 * K + 7 * N)
+    w = torch.randn(K, N, generator=g) / K**0.5
+    store = torch.randn(M * (K + 3) + 1, generator=g).half().to(dev)
+    a = {"plain": lambda: store[: M * K].view(M, K), "offset": lambda: store[1 : M * K + 1].view(M, K),
+         "wide_rows": lambda: store[: M * (K + 3)].view(M, K + 3)[:, 3:], "one_row": lambda: store[1 : K + 1].expand(M, K)}[a_form]()
+    ref = a.float().cpu() @ h16(w)
+    kw = {}
+    if epilogue:
+        bias, res = torch.randn(N, generator=g), torch.randn(M, N, generator=g)
+        ref = ref + h16(bias) + h16(res)
+        kw = {"bias": bias.half().to(dev), "residual": res.half().to(dev)}
+    y = cascaded_lowp_matmul(a, w.half().to(dev), **kw)
+    _lib.device_status()
+    assert y.shape == (M, N) and y.is_contiguous()
+    assert_close(y, ref, what=f"ragged {M}x{K}x{N} {a_form}")
