@@ -66,4 +66,29 @@ int launch_kernel(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
   return check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...), what);
 }
 
+// Clusters of `width` CTAs that can be resident at one time, for a kernel of which an SM holds one CTA.  Fewer than
+// SMs / width: a cluster stays inside one GPC, whose SM count need not be a multiple of the width.  Asked of the
+// runtime once per device and width (`cache`: one int per width up to 4, per device).
+template <typename Kernel>
+int resident_clusters(Kernel kernel, int threads, size_t smem, int width, int (*cache)[5]) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || width < 2 || width > 4) return sm_count() / width;
+  if (!cache[dev][width]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count() / width * width), cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = width, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr, cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = sm_count() / width;
+    }
+    cache[dev][width] = n < sm_count() / width ? n : sm_count() / width;
+  }
+  return cache[dev][width];
+}
+
 }  // namespace bxl

@@ -765,17 +765,22 @@ static int stages_for(int bn, int split, int pair = 0, int extra_smem = 0, int p
   return st;
 }
 
-// Pick the tile width, the K split and whether to pair CTAs, minimising a time model fitted
-// to a sweep of every (tile width, split, pairing) over the GEMM and convolution shapes of the
-// SDXL UNet on B200.  One CTA streams its operands at ~110 KB/us from L2 (the per-SM fill rate
-// bounds these kernels, not the tensor pipe), so a k-block of a 128 x bn tile costs
-// max(mma(bn), bytes / 110 KB/us) with bytes = 16 KB + bn*128 B.  A CTA pair moves half of the B
-// tile per CTA but its stage recycling crosses two SMs: 0.24 us + 0.63 ns * bn per k-block.
-// `a_min_us` is a floor per k-block for the A operand path (the multi-row image copies of the
-// convolution).  A wider tile or a pair moves fewer bytes per FLOP; a narrower tile or a K split
-// spreads the stream over more SMs when there are few tiles.
+static int g_clusters[64][5] = {};
+
+// Pick the tile width, the K split and whether to pair CTAs, minimising a time model fitted to a sweep of
+// every (tile width, split, pairing) over 110 GEMM and convolution shapes (2 to 32768 rows; both layouts of B;
+// strips; fp32 operands; the UNet's layers and random ones) on B200.  A k-block of a 128 x bn tile costs the
+// larger of its MMAs (0.256 us at 256 columns) and of its operand stream: 139 KB/us for one CTA; a pair, which
+// stages half of the B tile per CTA but recycles a stage across two SMs, 0.117 us + 0.643 ns * bn.
+// `a_min_us` is a floor per k-block for the A operand path (the multi-row image copies of the convolution).  A
+// wider tile or a pair moves fewer bytes per FLOP; a narrower tile or a K split spreads the stream over more
+// SMs when there are few tiles; `heavy` epilogues read a residual or write fp32.  Of near equals the wider tile
+// is taken.  The choice is on average 0.6 % slower than the best configuration of each shape (at most 10 %); the
+// constants before, fitted while issuing a copy cost several times as much, chose 2.2 % and up to 41 %, on the
+// UNet's own layers up to 28 % (conv 2 x 640 x 64 x 64: 65.6 -> 51.1 us; GEMM 2048 x 2560 x 640: 16.3 -> 13.3 us;
+// 32768 x 2560 x 640: 105.8 -> 92.5 us).
 static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int force_bn = 0, int force_split = 0,
-                               int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0, int parts = 1) {
+                               int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0, int parts = 1, bool heavy = false) {
   const int sms = sm_count();
   TileConfig best{128, 1, stages_for(128, 1, 0, extra_smem, parts), 0};
   double best_cost = 1e30;
@@ -792,16 +797,17 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
         const int st = stages_for(bn, split, pair, extra_smem, parts);
         if (st < 3) continue;
         const int width = pair ? 2 : split;
-        const int clusters = sms / width;
+        const int clusters = width > 1 ? resident_clusters(gemm_conv_kernel<false, false, true>, kGemmThreads, kSmemBudget, width, g_clusters) : sms;
         const int par = tiles < clusters ? tiles : clusters;
         const int rounds = (tiles + par - 1) / par;
         const double bytes = 16384.0 + bn * (pair ? 64.0 : 128.0);
-        const double kb_us = fmax(fmax((2 * parts - 1) * bn / 256.0 * 0.27, parts * (pair ? 0.24 + 0.00063 * bn : bytes / 110000.0)), a_min_us);
+        const double kb_us = fmax(fmax((2 * parts - 1) * bn / 256.0 * 0.256, parts * (pair ? 0.117 + 0.000643 * bn : bytes / 139000.0)), a_min_us);
         const double kb_unit = (num_kb + split - 1) / split;
-        const double epi_us = 0.08 * (bn / 32.0) / split + (split > 1 ? 1.2 : 0.0);  // accumulator read-out (+ exchange)
-        const double fill_us = 1.0 + (st < 4 ? 0.5 : 0.0) + (pair ? 0.3 : 0.0);       // pipeline ramp per unit
-        const double pair_tile_us = pair ? 0.45 : 0.0;  // accumulator hand-over between the two CTAs, per tile
-        const double cost = rounds * (kb_unit * kb_us + epi_us + pair_tile_us) + fill_us + 3.0;
+        // accumulator read-out (and the exchange of a K split)
+        const double epi_us = (heavy ? 0.455 : 0.271) * (bn / 32.0) / split + (split > 1 ? 3.23 : 0.0);
+        const double fill_us = 4.28 + (st < 4 ? 0.86 : 0.0);                       // launch, set-up and pipeline ramp
+        const double pair_tile_us = pair ? (heavy ? 1.014 : 0.67) : 0.0;           // accumulator hand-over between the two CTAs, per tile
+        const double cost = (rounds * (kb_unit * kb_us + epi_us + pair_tile_us) + fill_us) * (1.0 - 0.05 * bn / 256.0);
         if (cost < best_cost - 1e-9) {
           best_cost = cost;
           best = TileConfig{bn, split, st, pair};
@@ -846,7 +852,7 @@ static int aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 1
 
 // test hook: force the tile width / K split (0 = choose)
 constexpr int kDefaultPair = -1;  // -1 = let the cost model decide
-constexpr double kConvAMinUs = 0.36;  // per-k-block floor of the convolution's image copies
+constexpr double kConvAMinUs = 0.224;  // per-k-block floor of the convolution's image copies
 static int g_force_bn = 0, g_force_split = 0, g_force_pair = -1;
 static int g_force_order = -1;  // -1 = choose, 0 = consecutive tiles walk M, 1 = they walk N
 // Linear layers: an activation matrix that does not stay in L2 beside the output is walked once
@@ -876,7 +882,8 @@ extern "C" int bxl_gemm_f16(const void* A, long long lda, const void* B, long lo
   GemmParams p;
   memset(&p, 0, sizeof(p));
   const int tiles_m = (M + kBM - 1) / kBM;
-  const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, b_is_kn != 0, g_force_bn, g_force_split, g_force_pair < 0 ? kDefaultPair : g_force_pair);
+  const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, b_is_kn != 0, g_force_bn, g_force_split, g_force_pair < 0 ? kDefaultPair : g_force_pair,
+                                     0.0, 0, 1, residual != nullptr || out_f32);
   const int BN = tc.bn;
   {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
@@ -990,7 +997,7 @@ extern "C" int bxl_gemm_ragged_f16(const void* A, long long lda, const void* B, 
   const bool ragged = !aligned16(C) || ldc % 8 || N % 8 || (residual && (!aligned16(residual) || ldr % 8));
   const int tiles_m = (M + kBM - 1) / kBM;
   const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, true, g_force_bn, g_force_split,
-                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, ragged ? kSmemRaggedExtra : 0);
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, ragged ? kSmemRaggedExtra : 0, 1, ragged || residual);
   {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)M};
     uint64_t str[1] = {(uint64_t)a.ld_dst * 2};
@@ -1116,7 +1123,7 @@ extern "C" int bxl_gemm_fused_f16(const bxl_gemm_fused_args* a, int* row_stats_p
   memset(&p, 0, sizeof(p));
   const int tiles_m = (M + kBM - 1) / kBM;
   const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, false, g_force_bn, g_force_split,
-                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, ln ? kSmemLnExtra : 0);
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, ln ? kSmemLnExtra : 0, 1, a->residual != nullptr);
   const int tiles_n = (N + tc.bn - 1) / tc.bn;
   if (a->row_stats) {
     const long long parts = (long long)kEpiSub * tiles_n * (tc.pair ? 1 : tc.split);  // one per epilogue warp of a row and column slice
@@ -1229,7 +1236,7 @@ extern "C" int bxl_gemm_split_f32(const float* A, const float* B, float* C, int 
   memset(&p, 0, sizeof(p));
   const int tiles_m = (M + kBM - 1) / kBM;
   const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, true, g_force_bn, g_force_split,
-                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, 0, 2);
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, 0, 2, true);
   const int BN = tc.bn;
   // C = A_hi*B_hi + A_hi*B_lo + A_lo*B_hi, one fp32 accumulator.  The operand stream bounds the K loop, so a
   // ring slot holds the four parts of a k-block and three products are formed from it (four tiles copied for
