@@ -5,38 +5,37 @@
 // slot: the own strip's fresh K/V and the peers' stale K/V are never
 // concatenated.  The same kernel serves cross-attention (one slot, 77 tokens).
 //
-// Work unit = 256 queries (two tiles of 128) of one (image, head).  A CTA walks several units
-// (or, with a K/V split, a cluster of 2 or 4 CTAs shares one unit).  384 threads:
-//   warps 0..3  softmax group 0, warps 4..7 softmax group 1: thread r owns query row r of its
-//               tile (= TMEM lane r).  Per K/V tile it reads its row of S once (128 registers),
-//               releases S at once so the next Q K^T can start, takes the row maximum, forms
-//               P = exp2(S*scale - m) in fp32 (MUFU), sums the row in fp32 registers, packs P to
-//               fp16 and stores it to TENSOR MEMORY (tcgen05.st), from where the P V product
-//               reads it as its A operand: P never touches shared memory.  The running maximum
-//               m is only raised when the tile maximum exceeds it by more than 8 (a factor of
+// Work unit = up to 384 queries (three tiles of 128) of one (image, head).  A CTA walks several units
+// (or, with a K/V split, a cluster of 2 or 4 CTAs shares one unit).  512 threads:
+//   warps 0..11 three softmax groups of four warps: thread r of a group owns query row r of its
+//               tile (= TMEM lane r).  Per K/V tile (64 tokens) it reads its row of S once, releases S at
+//               once so the next Q K^T can start, takes the row maximum, forms P = exp2(S*scale - m) in
+//               fp32 (14 of 16 on the special-function unit, 2 on the FMA pipe), sums the row in fp32
+//               registers, packs P to fp16 and stores it to TENSOR MEMORY (tcgen05.st), from where the
+//               P V product reads it as its A operand: P never touches shared memory.  The running
+//               maximum m is only raised when the tile maximum exceeds it by more than 8 (a factor of
 //               256, harmless in fp16/fp32); only then O is rescaled in tensor memory
 //               (tcgen05.ld / multiply / tcgen05.st) and the row sum in its register.  The
 //               result is exact: O and the row sum always refer to the same m.
-//               These two warpgroups raise their register budget (setmaxnreg) at the expense
-//               of the third one.
-//   warp 8      TMA producer: the two Q tiles of a unit (double buffered across units), then a
-//               ring of {K tile, V tile} (128 tokens x 64) shared by the two query tiles
-//   warp 9      tensor memory owner and tcgen05.mma issuer (all 32 lanes run the loop, an
-//               elected lane issues), for the two query tiles g = 0, 1:
-//                 S_g  = Q_g K_j^T      (128x128, both operands K-major in shared memory)
-//                 O_g += P_g V_j        (128x64, P from tensor memory, V MN-major as stored)
-//               issued in the order in which their conditions come true.
-//   warps 10,11 idle (they complete the third warpgroup).
-// While one group runs its softmax the tensor core works for the other one; the K/V tiles of
+//               These warpgroups raise their register budget (setmaxnreg) at the expense of the last one.
+//   warp 12     TMA producer: the Q tiles of a unit (double buffered across units), then a
+//               ring of {K tile, V tile} (64 tokens x 64) shared by the query tiles
+//   warps 13..15 tcgen05.mma issuers, one per query tile; warp 13 owns tensor memory
+//
+// While one group runs its softmax the tensor core works for the others; the K/V tiles of
 // all units of a CTA form one stream, so the first Q K^T of the next unit and the read-out of
 // the finished unit's output overlap the unit boundary.
 //
-// Roofline: tensor cores; algorithmic FLOPs = 4 * L_q * L_kv * 64 per (image, head).
-// With head dimension 64 the softmax side (one MUFU exponential plus ~3 more instructions per
-// score, two warps per scheduler) needs more cycles per tile than the two matrix products;
-// measured, the kernel is bound by that instruction stream (evaluating part of the
-// exponentials with a polynomial on the FMA pipe made it slower).
-#include <stdlib.h>
+// Roofline: tensor cores; algorithmic FLOPs = 4 * L_q * L_kv * 64 per (image, head).  With head dimension 64
+// the exponentials (16 per clock and SM) are the narrowest resource, 1150 TFLOP/s at 1.9 GHz.  Counters at
+// 2 x 20 x 4096 x 4096: special-function unit 64 % busy, issue slots 54 %, tensor pipe 36 %: a softmax warp's
+// own dependences (read S, maximum, exponentials, publish P) bound it, so three warps per scheduler work
+// side by side where there were two with tiles of 128 tokens, and 384-query units leave fewer idle SMs in
+// the last round.  Measured (two groups of 128 x 128 tiles -> three of 128 x 64): 2 x 10 x 4096 x 4096
+// 167.8 -> 138.3 us, 2 x 20 x 4096 x 4096 257 -> 232 (741 TFLOP/s), 2 x 10 x 16384 x 16384 1886 -> 1851,
+// 2 x 20 x 1024 x 1024 29.3 -> 25.4, 1024 queries against 4 x 1024 keys 58.4 -> 46.5; 4096 queries against 77 keys
+// 13.3 -> 13.6, 16384 against 77 37.1 -> 30.5.  Exponentials on the FMA pipe: none 144.0 / 243 / 1880 us on the
+// first three shapes, 4 of 16 137.8 / 242 / 1878.
 
 #include "bxl_common.cuh"
 #include "bxl_host.h"
@@ -44,13 +43,21 @@
 
 namespace bxl {
 
-constexpr int kAttnThreads = 384;   // warps 0..7 softmax, 8 producer, 9 MMA issuer, 10..11 idle
-constexpr int kSoftmaxRegs = 208;   // registers per thread after the split: 8 x 32 x 208 + 4 x 32 x 88 = 64512
-constexpr int kOtherRegs = 88;
+constexpr int kGroups = 3;                         // softmax warpgroups = query tiles in flight
+constexpr int kWarpLoad = 4 * kGroups;             // producer warp; then one MMA issuer warp per group
+constexpr int kWarpMma = kWarpLoad + 1;
+constexpr int kAttnThreads = (4 * kGroups + 4) * 32;
+constexpr int kSoftmaxRegs = 144;   // registers per thread after the split: 12 x 32 x 144 + 4 x 32 x 80 = 512 x 128
+constexpr int kOtherRegs = 80;
+constexpr int kPolyOf16 = 2;        // score pairs of every 16 whose exponentials run on the FMA pipe
 constexpr int kHeadDim = 64;
 constexpr int kTileQ = 128;
-constexpr int kTileKV = 128;
-constexpr int kKvStages = 4;
+constexpr int kTileKV = 64;
+constexpr int kKvStages = 6;
+constexpr int kQBytes = kTileQ * kHeadDim * 2, kKvBytes = kTileKV * kHeadDim * 2;   // one Q tile; one K or V tile
+// tensor memory columns: S_g, O_g (fp32), P_g (two fp16 per column, the A operand of the P V product)
+constexpr int kTmemO = kGroups * kTileKV, kTmemP = kTmemO + kGroups * kHeadDim;
+static_assert(kTmemP + kGroups * kTileKV / 2 <= 512, "tensor memory");
 constexpr int kMaxSlots = 8;
 
 struct alignas(64) AttnParams {
@@ -64,15 +71,15 @@ struct alignas(64) AttnParams {
   long long out_img_stride, ld_out;
   float scale_log2e;               // softmax scale * log2(e)
   int kv_split;                    // K/V range split over a cluster of 1, 2 or 4 CTAs
-  int n_full;                      // units [0, n_full) are whole (256 queries); each later unit is served as two halves of 128
+  int groups;                      // query tiles per unit (1..kGroups)
   int* dev_status;
 };
 
 struct AttnSmem {
-  static constexpr int kQ = 0;                               // 2 buffers x 2 tiles x 16 KB
-  static constexpr int kK = 65536;                           // kKvStages x 16 KB
-  static constexpr int kV = kK + kKvStages * 16384;          // kKvStages x 16 KB
-  static constexpr int kBar = kV + kKvStages * 16384;
+  static constexpr int kQ = 0;                               // 2 buffers x kGroups tiles
+  static constexpr int kK = 2 * kGroups * kQBytes;
+  static constexpr int kV = kK + kKvStages * kKvBytes;
+  static constexpr int kBar = kV + kKvStages * kKvBytes;
   static constexpr int kTotal = kBar + 1024 + 1024;
 };
 
@@ -80,6 +87,77 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// Two fp32 values in one 64-bit register pair: one instruction for both (half the issue slots of the
+// softmax's multiply-adds and sums; the rounding is that of the scalar forms).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair2(f32x2 r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+// 2^x on the FMA pipe, for part of the scores: the special-function unit (16 results per clock and SM) is the
+// softmax's narrowest unit.  x = n + f with n the nearest integer (the sum with 1.5 * 2^23 + 127 leaves n + 127 in
+// the low mantissa bits), 2^f by a degree-5 polynomial fitted to |f| <= 0.5 for the smallest relative error
+// (2.1e-7 in fp32 arithmetic, the error bound of the special-function unit), times 2^n built from those bits.
+// x <= 8 here; below -120 the result is as good as zero; NaN stays NaN.
+__device__ __forceinline__ f32x2 poly_exp2(f32x2 x) {
+  float x0, x1;
+  unpair2(x, x0, x1);
+  x = pair2(max_nan(x0, -120.f), max_nan(x1, -120.f));
+  const float magic = 12582912.f + 127.f;
+  const f32x2 t = add2(x, pair2(magic, magic));
+  const f32x2 n = add2(t, pair2(-magic, -magic));
+  const f32x2 f = fma2(n, pair2(-1.f, -1.f), x);
+  f32x2 p = fma2(f, pair2(1.3276472454890609e-3f, 1.3276472454890609e-3f), pair2(9.675540961325169e-3f, 9.675540961325169e-3f));
+  p = fma2(p, f, pair2(5.550713092088699e-2f, 5.550713092088699e-2f));
+  p = fma2(p, f, pair2(2.4022120237350464e-1f, 2.4022120237350464e-1f));
+  p = fma2(p, f, pair2(6.931469440460205e-1f, 6.931469440460205e-1f));
+  p = fma2(p, f, pair2(1.f, 1.f));
+  float t0, t1;
+  unpair2(t, t0, t1);
+  return mul2(p, pair2(__uint_as_float(__float_as_uint(t0) << 23), __uint_as_float(__float_as_uint(t1) << 23)));
+}
+// P = 2^(s * scale - m) of two neighbouring scores: added to the row sum in fp32, packed to fp16.
+template <bool kPoly>
+__device__ __forceinline__ uint32_t exp_pair(uint32_t s0, uint32_t s1, f32x2 scale, f32x2 minus_m, f32x2& sum) {
+  const f32x2 x = fma2(pair2(__uint_as_float(s0), __uint_as_float(s1)), scale, minus_m);
+  float e0, e1;
+  f32x2 e;
+  if (kPoly) {
+    e = poly_exp2(x);
+    unpair2(e, e0, e1);
+  } else {
+    float x0, x1;
+    unpair2(x, x0, x1);
+    e0 = fast_exp2(x0), e1 = fast_exp2(x1);
+    e = pair2(e0, e1);
+  }
+  sum = add2(sum, e);
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(e1), "f"(e0));
+  return r;
 }
 __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
   uint32_t packed;
@@ -180,47 +258,43 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + AttnSmem::kBar;
-  // barriers: q_full[2], q_empty[2], kv_full[stages], kv_empty[stages], s_full[2], o_full[2], p_full[2], s_free[2]
+  // barriers: q_full[2], q_empty[2], kv_full[stages], kv_empty[stages], then per group s_full, o_full, p_full, s_free
   auto q_full = [&](int b) { return bar_base + 8u * b; };
   auto q_empty = [&](int b) { return bar_base + 8u * (2 + b); };
   auto kv_full = [&](int s) { return bar_base + 8u * (4 + s); };
   auto kv_empty = [&](int s) { return bar_base + 8u * (4 + kKvStages + s); };
-  auto s_full = [&](int g) { return bar_base + 8u * (4 + 2 * kKvStages + g); };
-  auto o_full = [&](int g) { return bar_base + 8u * (6 + 2 * kKvStages + g); };
-  auto p_full = [&](int g) { return bar_base + 8u * (8 + 2 * kKvStages + g); };
-  auto s_free = [&](int g) { return bar_base + 8u * (10 + 2 * kKvStages + g); };
+  constexpr int kGroupBar = 4 + 2 * kKvStages;
+  auto s_full = [&](int g) { return bar_base + 8u * (kGroupBar + g); };
+  auto o_full = [&](int g) { return bar_base + 8u * (kGroupBar + kGroups + g); };
+  auto p_full = [&](int g) { return bar_base + 8u * (kGroupBar + 2 * kGroups + g); };
+  auto s_free = [&](int g) { return bar_base + 8u * (kGroupBar + 3 * kGroups + g); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + AttnSmem::kBar + 512);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + AttnSmem::kBar + 520);
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  // S_0 [0,128) S_1 [128,256) O_0 [256,320) O_1 [320,384) P_0 [384,448) P_1 [448,512)
-  // (P: 128 fp16 per row packed two per 32-bit column, the A operand of the P V product)
   constexpr uint32_t kTmemCols = 512;
 
-  // Work units: 256 queries (two tiles) of one (image, head).
+  // Work units: up to `groups` query tiles of one (image, head).
   //   kv_split == 1: the CTA walks units blockIdx.x, blockIdx.x + gridDim.x, ...; barriers, the
   //     K/V ring and tensor memory live across units, Q is double buffered, so the loads and the
   //     first Q K^T of the next unit overlap the tail of the current one.
   //   kv_split == S > 1: the S CTAs of a cluster serve ONE unit, each over 1/S of the K/V tiles;
   //     their partial (max, sum, output) triples are merged through distributed shared memory at
-  //     the end (every CTA merges 256/S of the rows).
+  //     the end (every CTA merges 1/S of the rows).
   const int S = p.kv_split;
   const uint32_t crank = (S > 1) ? cluster_ctarank() : 0u;
-  const int q_pairs = (p.L_q + 2 * kTileQ - 1) / (2 * kTileQ);
-  // Units past n_full are the last, under-filled round of a persistent grid: each is served as two
-  // half units (one query tile) so that twice as many CTAs share that round.
-  const int n_full = p.n_full;
-  const int units_total = n_full + 2 * (q_pairs * p.heads * p.B - n_full);
+  const int unit_rows = p.groups * kTileQ;
+  const int q_units = (p.L_q + unit_rows - 1) / unit_rows;
+  const int units_total = q_units * p.heads * p.B;
   const int first_unit = (S > 1) ? static_cast<int>(blockIdx.x) / S : static_cast<int>(blockIdx.x);
   const int unit_step = (S > 1) ? units_total : static_cast<int>(gridDim.x);
-  auto unit_pair = [&](int w) { return w < n_full ? w : n_full + ((w - n_full) >> 1); };      // index of the 256-query block
-  auto unit_q_row0 = [&](int w) { return (unit_pair(w) % q_pairs) * 2 * kTileQ + ((w >= n_full && ((w - n_full) & 1)) ? kTileQ : 0); };
-  auto unit_head = [&](int w) { return (unit_pair(w) / q_pairs) % p.heads; };
-  auto unit_img = [&](int w) { return unit_pair(w) / (q_pairs * p.heads); };
-  // the second tile may lie wholly past L_q; a half unit has one tile
-  auto unit_groups = [&](int w) { return (w < n_full && unit_q_row0(w) + kTileQ < p.L_q) ? 2 : 1; };
+  auto unit_q_row0 = [&](int w) { return (w % q_units) * unit_rows; };
+  auto unit_head = [&](int w) { return (w / q_units) % p.heads; };
+  auto unit_img = [&](int w) { return w / (q_units * p.heads); };
+  // the last unit of a head may have fewer tiles
+  auto unit_groups = [&](int w) { return min(p.groups, (p.L_q - unit_q_row0(w) + kTileQ - 1) / kTileQ); };
   const int tiles_per_slot = (p.L_slot + kTileKV - 1) / kTileKV;
   const int total_tiles = p.n_slots * tiles_per_slot;
   const int tile0 = static_cast<int>((static_cast<long long>(crank) * total_tiles) / S);   // first K/V tile of this CTA
@@ -233,13 +307,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(q_full(b), 1);
-      mbar_init(q_empty(b), 1);
+      mbar_init(q_empty(b), kGroups);   // one arrival per issuer warp
     }
     for (int s = 0; s < kKvStages; ++s) {
       mbar_init(kv_full(s), 1);
-      mbar_init(kv_empty(s), 1);
+      mbar_init(kv_empty(s), kGroups);
     }
-    for (int g = 0; g < 2; ++g) {
+    for (int g = 0; g < kGroups; ++g) {
       mbar_init(s_full(g), 1);
       mbar_init(o_full(g), 1);
       mbar_init(p_full(g), 128);
@@ -248,7 +322,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 9) {
+  if (warp == kWarpMma) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
     tmem_relinquish();
   }
@@ -260,9 +334,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
   // producer / MMA warpgroup does not need
   pdl_wait();  // the set-up above overlaps the previous kernel's tail; global data from here on
 
-  if (warp >= 8) {
+  if (warp >= kWarpLoad) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
-  if (warp == 8) {
+  if (warp == kWarpLoad) {
     // ======================= TMA producer =======================
     // all 32 lanes run the loop (addresses stay warp-uniform); the elected lane issues
     const bool leader = elect_one();
@@ -279,171 +353,143 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       // the Q buffer was last used by unit ul - 2: all its Q K^T products must have completed
       if (ul >= 2 && !mbar_wait_warp(q_empty(qb), ((ul >> 1) - 1) & 1u, abort_flag, p.dev_status, 401)) break;
       if (leader) {
-        mbar_arrive_expect_tx(q_full(qb), 16384u * ng);
+        mbar_arrive_expect_tx(q_full(qb), static_cast<uint32_t>(kQBytes) * ng);
         for (int g = 0; g < ng; ++g)
-          tma_load_3d(smem_base + AttnSmem::kQ + qb * 32768 + g * 16384, &p.q_map, q_full(qb), head * kHeadDim,
+          tma_load_3d(smem_base + AttnSmem::kQ + (qb * kGroups + g) * kQBytes, &p.q_map, q_full(qb), head * kHeadDim,
                       q_row0 + g * kTileQ, img);
       }
       __syncwarp();
+      int slot = tile0 / tiles_per_slot, ts = tile0 % tiles_per_slot;
       for (int j = 0; j < n_tiles; ++j) {
-        const int slot = (tile0 + j) / tiles_per_slot;
-        const int t0 = ((tile0 + j) % tiles_per_slot) * kTileKV;
+        const int t0 = ts * kTileKV;
         if (!mbar_wait_warp(kv_empty(stage), phase ^ 1u, abort_flag, p.dev_status, 400)) {
           ok = false;
           break;
         }
         if (leader) {
-          mbar_arrive_expect_tx(kv_full(stage), 32768);
-          tma_load_3d(smem_base + AttnSmem::kK + stage * 16384, &p.kv_map[slot], kv_full(stage), head * kHeadDim, t0, img);
-          tma_load_3d(smem_base + AttnSmem::kV + stage * 16384, &p.kv_map[slot], kv_full(stage),
+          mbar_arrive_expect_tx(kv_full(stage), 2 * kKvBytes);
+          tma_load_3d(smem_base + AttnSmem::kK + stage * kKvBytes, &p.kv_map[slot], kv_full(stage), head * kHeadDim, t0, img);
+          tma_load_3d(smem_base + AttnSmem::kV + stage * kKvBytes, &p.kv_map[slot], kv_full(stage),
                       p.v_col0 + head * kHeadDim, t0, img);
         }
         __syncwarp();
+        if (++ts == tiles_per_slot) ts = 0, ++slot;
         if (++stage == kKvStages) {
           stage = 0;
           phase ^= 1u;
         }
       }
     }
-  } else if (warp == 9) {
-    // ======================= MMA issuer =======================
-    // all 32 lanes run the loop and the waits; the elected lane issues every tcgen05.mma and
-    // tcgen05.commit, so descriptors are formed from warp-uniform values.  The K/V tiles of all
-    // units of this CTA form one stream: while the softmax of tile t runs, Q K^T of tile t+1 is
-    // issued, also across a unit boundary.
+  } else {
+    // ======================= MMA issuers =======================
+    // One warp per query tile: its waits come true in a fixed order (S copied out, then P published), and
+    // a late group holds up nobody.  All 32 lanes run the loop and the waits; the elected lane issues
+    // every tcgen05.mma and tcgen05.commit, so descriptors are formed from warp-uniform values.  The K/V
+    // tiles of all units of this CTA form one stream: while the softmax of tile t runs, Q K^T of tile
+    // t + 1 is issued, also across a unit boundary.
+    const int g = warp - kWarpMma;
     const bool leader = elect_one();
-    const uint32_t idesc_s = make_idesc_f16(128, 128, 0, 0);  // S = Q K^T, both K-major
-    const uint32_t idesc_o = make_idesc_f16(128, 64, 0, 1);   // O = P V, V MN-major
-    int n_s[2] = {0, 0};   // Q K^T products issued per group (= phases of s_full started)
-    int n_pv[2] = {0, 0};  // P V products issued per group
-    int kv_t = 0;          // K/V tiles of the stream consumed so far
+    const uint32_t idesc_s = make_idesc_f16(kTileQ, kTileKV, 0, 0);   // S = Q K^T, both K-major
+    const uint32_t idesc_o = make_idesc_f16(kTileQ, kHeadDim, 0, 1);  // O = P V, V MN-major
+    int n_s = 0;     // Q K^T products issued (= phases of s_full started)
+    int n_pv = 0;    // P V products issued
+    int st = 0;      // ring stage and phase of the stream's current tile
+    uint32_t ph = 0;
+    bool s_issued = false;   // Q K^T of the current tile is already under way
     bool ok = true;
-    auto wait_kv = [&](int t) -> bool {
-      if (!mbar_wait_warp(kv_full(t % kKvStages), (t / kKvStages) & 1u, abort_flag, p.dev_status, 501)) return false;
+    // S_g = Q_g K^T for the tile in ring stage `stage`; S_g must have been read by the softmax group if it
+    // was ever written
+    auto issue_s = [&](int qb, int stage, uint32_t phase) -> bool {
+      if (!mbar_wait_warp(kv_full(stage), phase, abort_flag, p.dev_status, 501)) return false;
+      if (n_s > 0 && !mbar_wait_warp(s_free(g), (n_s - 1) & 1u, abort_flag, p.dev_status, 503)) return false;
       tc_fence_after_sync();
-      return true;
-    };
-    // S_g = Q_g K^T for stream tile t of the unit in Q buffer qb; S_g must have been read by the
-    // softmax group (s_free) if it was ever written
-    auto issue_s = [&](int qb, int g, int t) -> bool {
-      if (n_s[g] > 0) {
-        if (!mbar_wait_warp(s_free(g), (n_s[g] - 1) & 1u, abort_flag, p.dev_status, 503)) return false;
-        tc_fence_after_sync();
-      }
-      const int st = t % kKvStages;
-      const uint64_t qdesc = make_smem_desc_sw128(smem_base + AttnSmem::kQ + qb * 32768 + g * 16384, 16, 1024);
-      const uint64_t kdesc = make_smem_desc_sw128(smem_base + AttnSmem::kK + st * 16384, 16, 1024);
-      const uint32_t d = tmem_base + g * 128;
+      const uint64_t qdesc = make_smem_desc_sw128(smem_base + AttnSmem::kQ + (qb * kGroups + g) * kQBytes, 16, 1024);
+      const uint64_t kdesc = make_smem_desc_sw128(smem_base + AttnSmem::kK + stage * kKvBytes, 16, 1024);
       if (leader) {
 #pragma unroll
-        for (int k = 0; k < kHeadDim / 16; ++k) umma_f16(d, qdesc + 2u * k, kdesc + 2u * k, idesc_s, k != 0);
+        for (int k = 0; k < kHeadDim / 16; ++k) umma_f16(tmem_base + g * kTileKV, qdesc + 2u * k, kdesc + 2u * k, idesc_s, k != 0);
         umma_commit(s_full(g));
       }
       __syncwarp();
-      ++n_s[g];
+      ++n_s;
       return true;
     };
     int ul = 0;
-    if (first_unit < units_total) {
-      // first tile of the first unit
-      ok = mbar_wait_warp(q_full(0), 0, abort_flag, p.dev_status, 500) && wait_kv(0);
-      for (int g = 0; g < unit_groups(first_unit) && ok; ++g) ok = issue_s(0, g, 0);
-    }
     for (int w = first_unit; w < units_total && ok; w += unit_step, ++ul) {
       const int qb = ul & 1;
-      const int ng = unit_groups(w);
+      const bool active = g < unit_groups(w);
       const int w_next = w + unit_step;
-      const bool has_next_unit = w_next < units_total;
-      for (int j = 0; j < n_tiles && ok; ++j, ++kv_t) {
-        const int st = kv_t % kKvStages;
-        // tokens of this tile that exist (the last tile of a slot may be ragged): P is zero beyond
-        // them, so their 16-token steps of the P V product are skipped
-        const int k_steps = (min(kTileKV, p.L_slot - ((tile0 + j) % tiles_per_slot) * kTileKV) + 15) / 16;
-        // V tile [128 tokens][64] as stored: MN-major B operand, 8-token groups 1 KB apart
-        const uint64_t vdesc = make_smem_desc_sw128(smem_base + AttnSmem::kV + st * 16384, 16, 1024);
-        // the tile after this one in the stream
-        int nxt_ng = 0, nxt_qb = qb;
-        if (j + 1 < n_tiles) {
-          nxt_ng = ng;
+      const bool next_active = w_next < units_total && g < unit_groups(w_next);
+      if (!s_issued && !mbar_wait_warp(q_full(qb), (ul >> 1) & 1u, abort_flag, p.dev_status, 500)) {
+        ok = false;
+        break;
+      }
+      if (!active && leader) mbar_arrive(q_empty(qb));
+      int ts = tile0 % tiles_per_slot;
+      for (int j = 0; j < n_tiles; ++j) {
+        int st_next = st + 1;
+        uint32_t ph_next = ph;
+        if (st_next == kKvStages) st_next = 0, ph_next ^= 1u;
+        if (!active) {
+          // the ring stage is released by all issuers, in step with its phases
+          if (!mbar_wait_warp(kv_full(st), ph, abort_flag, p.dev_status, 504)) {
+            ok = false;
+            break;
+          }
+          if (leader) mbar_arrive(kv_empty(st));
+          __syncwarp();
         } else {
-          // every Q K^T of this unit has been issued: its Q buffer is free once they complete
-          if (leader) umma_commit(q_empty(qb));
-          __syncwarp();
-          if (has_next_unit) {
-            nxt_ng = unit_groups(w_next), nxt_qb = qb ^ 1;
-            if (!mbar_wait_warp(q_full(nxt_qb), ((ul + 1) >> 1) & 1u, abort_flag, p.dev_status, 500)) {
+          if (!s_issued && !issue_s(qb, st, ph)) {
+            ok = false;
+            break;
+          }
+          s_issued = false;
+          if (j + 1 < n_tiles) {
+            if (!issue_s(qb, st_next, ph_next)) {
               ok = false;
               break;
             }
+            s_issued = true;
+          } else {
+            // every Q K^T of this unit has been issued: its Q buffer is free once they complete
+            if (leader) umma_commit(q_empty(qb));
+            __syncwarp();
+            if (next_active) {
+              if (!mbar_wait_warp(q_full(qb ^ 1), ((ul + 1) >> 1) & 1u, abort_flag, p.dev_status, 500) || !issue_s(qb ^ 1, st_next, ph_next)) {
+                ok = false;
+                break;
+              }
+              s_issued = true;
+            }
           }
-        }
-        if (nxt_ng > 0 && !wait_kv(kv_t + 1)) {
-          ok = false;
-          break;
-        }
-        // Four things are due for this tile: Q K^T of the next tile (per group, once the group
-        // has copied its S) and P V of this tile (per group, once its P is published).  They are
-        // issued in the order in which their conditions come true, so a late group never holds
-        // up the other one.
-        bool due_s[2] = {nxt_ng > 0, nxt_ng > 1};
-        bool due_pv[2] = {ng > 0, ng > 1};
-        const unsigned long long t_start = global_timer_ns();
-        uint32_t spins = 0;
-        while (due_s[0] || due_s[1] || due_pv[0] || due_pv[1]) {
-          bool progress = false;
+          // P_g of this tile is in tensor memory; O_g carries the right scale
+          if (!mbar_wait_warp(p_full(g), n_pv & 1u, abort_flag, p.dev_status, 502)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          // tokens of this tile that exist (the last tile of a slot may be ragged): P is zero beyond
+          // them, so their 16-token steps of the P V product are skipped
+          const int k_steps = (min(kTileKV, p.L_slot - ts * kTileKV) + 15) / 16;
+          // V tile [64 tokens][64] as stored: MN-major B operand, 8-token groups 1 KB apart
+          const uint64_t vdesc = make_smem_desc_sw128(smem_base + AttnSmem::kV + st * kKvBytes, 16, 1024);
+          if (leader) {
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            if (due_s[g]) {
-              const bool ready = (n_s[g] == 0) || __all_sync(0xffffffffu, mbar_try_wait(s_free(g), (n_s[g] - 1) & 1u));
-              if (ready) {
-                ok = issue_s(nxt_qb, g, kv_t + 1);  // its own wait on s_free returns at once
-                due_s[g] = false, progress = true;
-              }
+            for (int k = 0; k < kTileKV / 16; ++k) {
+              // tokens 16k..16k+15: 8 packed columns of P, V rows advance by 16 x 128 B
+              if (k < k_steps)
+                umma_f16_ts(tmem_base + kTmemO + g * kHeadDim, tmem_base + kTmemP + g * (kTileKV / 2) + 8u * k, vdesc + 128u * k, idesc_o,
+                            (j != 0) | k);
             }
-            if (due_pv[g] && __all_sync(0xffffffffu, mbar_try_wait(p_full(g), n_pv[g] & 1u))) {
-              // P_g of this tile is in tensor memory; O_g carries the right scale
-              tc_fence_after_sync();
-              const uint32_t d = tmem_base + 256 + g * 64;
-              const uint32_t pt = tmem_base + 384 + g * 64;
-              const uint32_t acc = (j != 0);
-              if (leader) {
-#pragma unroll
-                for (int k = 0; k < kTileKV / 16; ++k) {
-                  // tokens 16k..16k+15: 8 packed columns of P, V rows advance by 16 x 128 B
-                  if (k < k_steps) umma_f16_ts(d, pt + 8u * k, vdesc + 128u * k, idesc_o, acc | k);
-                }
-                umma_commit(o_full(g));
-              }
-              __syncwarp();
-              ++n_pv[g];
-              due_pv[g] = false, progress = true;
-            }
+            umma_commit(o_full(g));
+            // K and V of this tile are no longer needed by this group once everything issued so far has completed
+            umma_commit(kv_empty(st));
           }
-          if (!ok) break;
-          if (!progress && (++spins & 63u) == 0u) {
-            // bounded: give up after the common wait limit and report where
-            bool give_up = (*abort_flag != 0);
-            if (!give_up && global_timer_ns() - t_start > kWaitLimitNs) {
-              give_up = true;
-              *abort_flag = 1;
-              if (atomicCAS(&p.dev_status[0], kDevOk, kDevWaitTimeout) == kDevOk) {
-                p.dev_status[1] = 502;
-                p.dev_status[2] = static_cast<int>(blockIdx.x);
-              }
-              __threadfence();
-            }
-            if (__any_sync(0xffffffffu, give_up)) {
-              ok = false;
-              break;
-            }
-          }
-        }
-        if (!ok) break;
-        // K and V of this tile are no longer needed once everything issued so far has completed
-        if (ok) {
-          if (leader) umma_commit(kv_empty(st));
           __syncwarp();
+          ++n_pv;
         }
+        if (++ts == tiles_per_slot) ts = 0;
+        st = st_next, ph = ph_next;
       }
     }
   }
@@ -455,15 +501,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       cluster_sync_all();
     }
   } else {
-    // ======================= softmax / output (warps 0..7) =======================
+    // ======================= softmax / output (warps 0..11) =======================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
     const int g = warp >> 2;               // query tile served by this warp
     const int quarter = warp & 3;          // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;   // query row inside the tile == TMEM lane
     const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t s_addr = t_lane + g * 128;
-    const uint32_t o_addr = t_lane + 256 + g * 64;
-    const uint32_t p_addr = t_lane + 384 + g * 64;
+    const uint32_t s_addr = t_lane + g * kTileKV;
+    const uint32_t o_addr = t_lane + kTmemO + g * kHeadDim;
+    const uint32_t p_addr = t_lane + kTmemP + g * (kTileKV / 2);
     const float sc = p.scale_log2e;
     constexpr float kRaise = 8.f;  // raise m only when the tile maximum exceeds it by 2^8
     int cnt = 0;                   // K/V tiles this group has processed (all units)
@@ -490,9 +536,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       if (g >= unit_groups(w)) continue;
       float m_run = -INFINITY;   // running row maximum in the exp2 domain (score * scale * log2 e)
       float l_run = 0.f;         // running row sum of P, same reference as O
+      int ts = tile0 % tiles_per_slot;
       for (int j = 0; j < n_tiles && ok; ++j, ++cnt) {
-        const int t0 = ((tile0 + j) % tiles_per_slot) * kTileKV;
-        const int valid = min(kTileKV, p.L_slot - t0);
+        const int valid = min(kTileKV, p.L_slot - ts * kTileKV);
+        if (++ts == tiles_per_slot) ts = 0;
         if (!mbar_wait(s_full(g), cnt & 1u, abort_flag, p.dev_status, 600)) {
           ok = false;
           break;
@@ -500,11 +547,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         __syncwarp();
         tc_fence_after_sync();
         // the whole row of S into registers, then hand the buffer back
-        uint32_t v0[32], v1[32], v2[32], v3[32];
+        uint32_t v0[32], v1[32];
         tmem_ld_32x32(s_addr, v0);
         tmem_ld_32x32(s_addr + 32, v1);
-        tmem_ld_32x32(s_addr + 64, v2);
-        tmem_ld_32x32(s_addr + 96, v3);
         tmem_ld_wait();
         tc_fence_before_sync();
         mbar_arrive(s_free(g));
@@ -513,16 +558,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         if (valid == kTileKV) {
           float ma = -INFINITY, mb = -INFINITY, mc = -INFINITY, md = -INFINITY;
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
+          for (int i = 0; i < 32; i += 4) {
             ma = max3(ma, __uint_as_float(v0[i]), __uint_as_float(v0[i + 1]));
             mb = max3(mb, __uint_as_float(v1[i]), __uint_as_float(v1[i + 1]));
-            mc = max3(mc, __uint_as_float(v2[i]), __uint_as_float(v2[i + 1]));
-            md = max3(md, __uint_as_float(v3[i]), __uint_as_float(v3[i + 1]));
+            mc = max3(mc, __uint_as_float(v0[i + 2]), __uint_as_float(v0[i + 3]));
+            md = max3(md, __uint_as_float(v1[i + 2]), __uint_as_float(v1[i + 3]));
           }
           m_tile = fmaxf(fmaxf(ma, mb), fmaxf(mc, md));
         } else {
-          m_tile = fmaxf(fmaxf(ragged_chunk_max(v0, valid), ragged_chunk_max(v1, valid - 32)),
-                         fmaxf(ragged_chunk_max(v2, valid - 64), ragged_chunk_max(v3, valid - 96)));
+          m_tile = fmaxf(ragged_chunk_max(v0, valid), ragged_chunk_max(v1, valid - 32));
         }
         const float m_new = fmaxf(m_run, m_tile * sc);
         float alpha = 1.f;
@@ -534,27 +578,28 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         }
         const bool rescale = __any_sync(0xffffffffu, alpha != 1.f);
         // P = exp2(S*scale - m) in fp32, summed in fp32, packed to fp16 for the tensor core:
-        // pa = columns [0,64), pb = columns [64,128), two per 32-bit word
-        uint32_t pa[32], pb[32];
-        float sum0 = 0.f, sum1 = 0.f, sum2 = 0.f, sum3 = 0.f;
+        // two per 32-bit word
+        uint32_t pa[32];
+        float sum0, sum1;
         if (valid == kTileKV) {
+          const f32x2 sc2 = pair2(sc, sc), nm2 = pair2(-m_run, -m_run);
+          f32x2 q0 = pair2(0.f, 0.f), q1 = q0;
+          // spread evenly over the row, so that both units stay busy
+          auto on_fma = [](int k) { return (k * kPolyOf16) / 16 != ((k + 1) * kPolyOf16) / 16; };
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float a0 = fast_exp2(fmaf(__uint_as_float(v0[2 * i]), sc, -m_run)), a1 = fast_exp2(fmaf(__uint_as_float(v0[2 * i + 1]), sc, -m_run));
-            const float b0 = fast_exp2(fmaf(__uint_as_float(v1[2 * i]), sc, -m_run)), b1 = fast_exp2(fmaf(__uint_as_float(v1[2 * i + 1]), sc, -m_run));
-            const float c0 = fast_exp2(fmaf(__uint_as_float(v2[2 * i]), sc, -m_run)), c1 = fast_exp2(fmaf(__uint_as_float(v2[2 * i + 1]), sc, -m_run));
-            const float d0 = fast_exp2(fmaf(__uint_as_float(v3[2 * i]), sc, -m_run)), d1 = fast_exp2(fmaf(__uint_as_float(v3[2 * i + 1]), sc, -m_run));
-            sum0 += a0 + a1, sum1 += b0 + b1, sum2 += c0 + c1, sum3 += d0 + d1;
-            pa[i] = pack_f16x2(a0, a1), pa[16 + i] = pack_f16x2(b0, b1), pb[i] = pack_f16x2(c0, c1), pb[16 + i] = pack_f16x2(d0, d1);
+            pa[i] = on_fma(2 * i) ? exp_pair<true>(v0[2 * i], v0[2 * i + 1], sc2, nm2, q0) : exp_pair<false>(v0[2 * i], v0[2 * i + 1], sc2, nm2, q0);
+            pa[16 + i] = on_fma(2 * i + 1) ? exp_pair<true>(v1[2 * i], v1[2 * i + 1], sc2, nm2, q1) : exp_pair<false>(v1[2 * i], v1[2 * i + 1], sc2, nm2, q1);
           }
+          float u0, u1;
+          unpair2(q0, u0, u1), sum0 = u0 + u1;
+          unpair2(q1, u0, u1), sum1 = u0 + u1;
         } else {
           // ragged last tile of a slot: columns >= valid contribute nothing
           sum0 = ragged_chunk_p<0>(v0, pa, valid, sc, m_run);
           sum1 = ragged_chunk_p<16>(v1, pa, valid - 32, sc, m_run);
-          sum2 = ragged_chunk_p<0>(v2, pb, valid - 64, sc, m_run);
-          sum3 = ragged_chunk_p<16>(v3, pb, valid - 96, sc, m_run);
         }
-        l_run = fmaf(l_run, alpha, (sum0 + sum1) + (sum2 + sum3));
+        l_run = fmaf(l_run, alpha, sum0 + sum1);
         // the previous P V product of this group must have finished: it read the P buffer, and O
         // is only touched between two products
         if (j == 0) {
@@ -585,7 +630,6 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         }
         // publish P in tensor memory
         tmem_st_32x32(p_addr, pa);
-        tmem_st_32x32(p_addr + 32, pb);
         tmem_st_wait();
         tc_fence_before_sync();
         mbar_arrive(p_full(g));
@@ -618,13 +662,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
     if (S > 1) {
       const int w = first_unit;
       const int n_groups = unit_groups(w);
-      const bool softmax_thread = (warp < 8) && ((warp >> 2) < n_groups);
+      const bool softmax_thread = (warp >> 2) < n_groups;
       const int sg = warp >> 2, srow = (warp & 3) * 32 + lane;     // group and row of a softmax thread
-      const int grow = sg * kTileQ + srow;                                 // row within the unit's 256 queries
+      const int grow = sg * kTileQ + srow;                                 // row within the unit's queries
       // every CTA of the cluster has left its K/V loop: the K/V ring of each CTA is free and serves
       // as the receive buffer  [sender][66 values][rows owned] (fp32)
       cluster_sync_all();
-      const int rows_owned = 2 * kTileQ / S;
+      const int rows_owned = unit_rows / S;
       const uint32_t owner = softmax_thread ? static_cast<uint32_t>(grow / rows_owned) : 0u;
       const int lrow = grow % rows_owned;
       const uint32_t recv = smem_base + AttnSmem::kK;
@@ -679,15 +723,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
     while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 9) {
+  if (warp == kWarpMma) {
     __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
+static int g_attn_clusters[64][5] = {};
 static int g_force_attn_split = 0;  // test hook: 0 = choose
-static int g_attn_tail_split = 1;   // serve an under-filled last round as half units (BXL_ATTN_TAIL_SPLIT=0 turns it off)
 
 }  // namespace bxl
 
@@ -744,36 +788,30 @@ extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long
       return rc;
     configured[dev] = true;
   }
-  const int q_pairs = (L_q + 2 * kTileQ - 1) / (2 * kTileQ);
-  const int work = q_pairs * heads * B;
+  // Query tiles per unit and K/V split: fewest rounds x time of a round, in K/V tiles of a full unit (1.2 us).  A
+  // unit of fewer query tiles takes not much less time (its softmax warps then share the special-function units
+  // with fewer others), it only fills more CTAs.  Without a split a CTA walks several units and pays ~1.5 tiles of
+  // bubble per unit; with a split each cluster serves one unit and pays ~6.5 tiles of set-up and merge.  Over 20
+  // shapes (64 to 16384 queries, 77 to 16384 keys) the choice is the fastest of the nine combinations or within 4 %.
+  const int q_tiles = (L_q + kTileQ - 1) / kTileQ;
   const int total_tiles = n_slots * ((L_slot + kTileKV - 1) / kTileKV);
-  // K/V split: fewest rounds x tiles per round.  Without a split a CTA walks several units and
-  // pays ~1 tile of bubble per unit plus ~2.5 once; with a split each cluster serves one unit and
-  // pays ~2.5 tiles of set-up and ~1.5 for the merge.
-  int split = 1;
+  static const double kTileCost[kGroups + 1] = {0.0, 0.58, 0.85, 1.0};
+  int split = 1, groups = kGroups;
   double best = 1e30;
-  for (int s2 = 1; s2 <= 4; s2 *= 2) {
-    if (s2 > total_tiles || (g_force_attn_split && s2 != g_force_attn_split)) continue;
-    const int clusters = sm_count() / s2;
-    const int rounds = (work + clusters - 1) / clusters;
-    const double cost = (s2 == 1) ? rounds * (total_tiles + 1.0) + 2.5 : rounds * ((total_tiles + s2 - 1) / s2 + 2.5 + 1.5);
-    if (cost < best - 1e-9) best = cost, split = s2;
+  for (int g = kGroups; g >= 1; --g) {
+    const int work = ((q_tiles + g - 1) / g) * heads * B;
+    for (int s2 = 1; s2 <= 4; s2 *= 2) {
+      if (s2 > total_tiles || (g_force_attn_split && s2 != g_force_attn_split)) continue;
+      const int clusters = s2 > 1 ? resident_clusters(attention_kernel, kAttnThreads, AttnSmem::kTotal, s2, g_attn_clusters) : sm_count();
+      const int rounds = (work + clusters - 1) / clusters;
+      const double tc = kTileCost[g < q_tiles ? g : (q_tiles < kGroups ? q_tiles : kGroups)];
+      const double cost = (s2 == 1) ? rounds * (total_tiles * tc + 1.5) : rounds * (((total_tiles + s2 - 1) / s2) * tc + 6.5);
+      if (cost < best - 1e-9) best = cost, split = s2, groups = g;
+    }
   }
-  p.kv_split = split;
-  // A persistent grid whose last round would keep at most half of the SMs busy serves that round's
-  // units as half units (one query tile each): twice the CTAs, about half the time.
-  p.n_full = work;
-  static int tail_env = -1;
-  if (tail_env < 0) {
-    const char* e = getenv("BXL_ATTN_TAIL_SPLIT");
-    tail_env = (e && e[0] == '0') ? 0 : 1;
-  }
-  if (split == 1 && g_attn_tail_split && tail_env && L_q % (2 * kTileQ) == 0 && work > sm_count()) {
-    const int rem = work % sm_count();
-    if (rem > 0 && 2 * rem <= sm_count()) p.n_full = work - rem;
-  }
-  const int units = p.n_full + 2 * (work - p.n_full);
-  const int grid = (split == 1) ? (units < sm_count() ? units : sm_count()) : work * split;
+  p.kv_split = split, p.groups = groups;
+  const int work = ((q_tiles + groups - 1) / groups) * heads * B;
+  const int grid = (split == 1) ? (work < sm_count() ? work : sm_count()) : work * split;
   return launch_kernel("attention_kernel launch", attention_kernel, dim3(grid), dim3(kAttnThreads), AttnSmem::kTotal,
                        (cudaStream_t)stream, split, p);
 }

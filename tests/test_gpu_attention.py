@@ -160,3 +160,64 @@ def test_self_attention_at_16384_tokens():
     y = ops.attention(q[:, i * ls : (i + 1) * ls].half().to(dev), [s.half().to(dev).contiguous() for s in slots], heads)
     _lib.device_status()
     assert_close(y, ref, what="self-attention L=16384")
+
+
+@pytest.mark.parametrize("split", [0, 1, 2])
+@pytest.mark.parametrize("Lq", [1, 128, 129, 257, 384, 385, 513, 770])
+@pytest.mark.parametrize("Lslot,nslots", [(1, 3), (63, 1), (64, 2), (65, 2), (200, 8)])
+def test_attention_tile_edges(Lq, Lslot, nslots, split):
+    """One to three query tiles per unit with the last one ragged, key tiles that end on, before and after a
+    64-token boundary, and more than one ring's worth of them."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    B, heads = 2, 3
+    C = heads * 64
+    gen = torch.Generator().manual_seed(Lq + 1000 * Lslot + nslots)
+    q = h16(torch.randn(B, Lq, C, generator=gen))
+    slots = [h16(torch.randn(B, Lslot, 2 * C, generator=gen)) for _ in range(nslots)]
+    ref = po._sdpa_heads(q, torch.cat(slots, dim=1), heads)
+    l = _lib.lib()
+    _lib.check(l.bxl_debug_force_attn_split(split), l, kernels=0)
+    try:
+        y = ops.attention(q.half().to(dev), [s.half().to(dev) for s in slots], heads)
+        _lib.device_status()
+    finally:
+        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
+    assert_close(y, ref, what=f"attention Lq{Lq} Ls{Lslot} n{nslots} split{split}")
+
+
+def test_attention_walks_many_units():
+    """More units than CTAs, the last unit of every head with one tile: the groups' barriers and the rings of
+    keys and queries go round many times, with idle groups in between."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    B, heads, Lq, Lslot = 2, 20, 4 * 384 + 60, 150
+    C = heads * 64
+    gen = torch.Generator().manual_seed(9)
+    q, kv = h16(torch.randn(B, Lq, C, generator=gen)), h16(torch.randn(B, Lslot, 2 * C, generator=gen))
+    ref = po._sdpa_heads(q, kv, heads)
+    l = _lib.lib()
+    _lib.check(l.bxl_debug_force_attn_split(1), l, kernels=0)
+    try:
+        y = ops.attention(q.half().to(dev), [kv.half().to(dev)], heads)
+        _lib.device_status()
+    finally:
+        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
+    assert_close(y, ref, what="attention, many units")
+
+
+def test_attention_keeps_nan_and_infinite_scores():
+    """A NaN in one key makes every row NaN, and a key of infinite score as well (inf - inf); other heads are
+    untouched."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    gen = torch.Generator().manual_seed(10)
+    q, kv = torch.randn(1, 200, 128, generator=gen).abs().half(), torch.randn(1, 320, 256, generator=gen).half()
+    clean = ops.attention(q.to(dev), [kv.to(dev)], 2)
+    for value, token in [(float("nan"), t) for t in range(64, 96)] + [(float("inf"), 70)]:
+        bad = kv.clone()
+        bad[0, token, 5] = value
+        y = ops.attention(q.to(dev), [bad.to(dev)], 2)
+        assert torch.isnan(y[..., :64]).all(), (value, token)
+        assert torch.equal(y[..., 64:], clean[..., 64:])
+    _lib.device_status()
