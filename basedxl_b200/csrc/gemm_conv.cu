@@ -273,18 +273,26 @@ __device__ __forceinline__ void store_chunk_ragged(const GemmParams& p, const fl
   }
 }
 
+// Accumulators of one tile.  The tensor core truncates its fp32 sums, by an amount that follows the sum's size and the
+// number of additions to it.  The split-operand product therefore adds its two small products (hi*lo and lo*hi, 2^-11
+// of hi*hi) to an accumulator of their own, and hi*hi, where the tile is narrow enough, to three over successive parts of
+// the K range; the epilogue adds them in fp32.  Error against 64 bits at K = 640: 3.4e-6 with one accumulator, 0.8e-6 so.
+__host__ __device__ inline int acc_sets(int parts, int bn) { return parts == 1 ? 1 : bn <= 64 ? 4 : 2; }
+
 // kSplit: the K loop is split over the CTAs of a cluster (p.split of them); a separate
 // instantiation, so that each variant carries only its own epilogue (and its registers).
-template <bool kConv, bool kPair, bool kSplit>
+// kTwo: operands in two fp16 parts (p.parts == 2); likewise separate.
+template <bool kConv, bool kPair, bool kSplit, bool kTwo>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid_constant__ GemmParams p) {
   static_assert(!(kPair && kSplit), "a CTA pair walks the whole K range");
+  static_assert(!(kConv && kTwo), "convolutions have fp16 operands");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int BN = p.bn;
   const int S = kSplit ? p.split : 1;
   const int b_rows = kPair ? BN / 2 : BN;       // rows of the B tile this CTA stages
-  const int parts = kConv ? 1 : p.parts;
+  constexpr int parts = kTwo ? 2 : 1;
   const int b_bytes = b_rows * 128;
   const int stage_bytes = parts * (kABytes + b_bytes);   // every part of A, then every part of B
   constexpr int kWidth = kPair ? 2 : 1;          // CTAs that cooperate on one tile (besides a K split)
@@ -308,7 +316,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t tmem_cols = (2 * BN <= 64) ? 64u : (2 * BN <= 128) ? 128u : (2 * BN <= 256) ? 256u : 512u;
+  const int sets = acc_sets(parts, BN);
+  const int acc_cols = sets * BN;   // tensor memory columns of one of the two accumulator buffers
+  const uint32_t tmem_cols = (2 * acc_cols <= 64) ? 64u : (2 * acc_cols <= 128) ? 128u : (2 * acc_cols <= 256) ? 256u : 512u;
   const uint32_t crank = (S > 1 || kPair) ? cluster_ctarank() : 0u;
 
   if (threadIdx.x == 0) {
@@ -358,6 +368,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
   const uint32_t krank = kPair ? 0u : crank;  // both CTAs of a pair walk the whole K range
   const int kb_begin = static_cast<int>((static_cast<long long>(krank) * num_kb) / S);
   const int kb_end = static_cast<int>((static_cast<long long>(krank + 1) * num_kb) / S);
+  const int main_sets = sets > 1 ? min(sets - 1, kb_end - kb_begin) : 1;   // accumulators of hi*hi, each over at least one k-block
   const int first_tile = blockIdx.x / (S * kWidth);
   const int tile_step = gridDim.x / (S * kWidth);
 
@@ -494,7 +505,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
                   : !mbar_wait(tempty_bar(acc), acc_phase ^ 1u, abort_flag, p.dev_status, 200))
           break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * acc_cols;
+        int set = 0, set_end = kb_begin + (kb_end - kb_begin) / main_sets;   // hi*hi: this accumulator's last k-block + 1
         for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (kPair ? !mbar_wait_cluster(full_bar(stage), phase, abort_flag, p.dev_status, 201)
                     : !mbar_wait(full_bar(stage), phase, abort_flag, p.dev_status, 201)) {
@@ -509,14 +521,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
           if (!kConv && p.b_kn) {
             // MN-major B: 64-column chunks 8 KB apart (LBO), 8-row k-groups 1 KB apart (SBO)
             const uint64_t bdesc = make_smem_desc_sw128(b_addr, 8192, 1024);
-            // split operands: hi*hi, hi*lo, lo*hi into the same accumulator, each part staged once
+            // split operands: hi*hi, hi*lo, lo*hi, each part staged once
+            uint32_t fresh = first;
+            if (kTwo && kb == set_end) {
+              ++set, fresh = 0u;
+              set_end = kb_begin + static_cast<int>((static_cast<long long>(set + 1) * (kb_end - kb_begin)) / main_sets);
+            }
             for (int t = 0; t < 2 * parts - 1; ++t) {
               const uint64_t ad = adesc + (t == 2 ? kABytes / 16 : 0);
               const uint64_t bd = bdesc + (t == 1 ? b_bytes / 16 : 0);
+              const uint32_t d = d_tmem + (t == 0 ? set : sets - 1) * BN;
+              const uint32_t add = t == 0 ? fresh : t == 1 ? first : 1u;
 #pragma unroll
               for (int k = 0; k < kBK / kUmmaK; ++k) {
-                if (kPair) umma_f16_pair(d_tmem, ad + 2u * k, bd + 128u * k, idesc, first | k | t);
-                else umma_f16(d_tmem, ad + 2u * k, bd + 128u * k, idesc, first | k | t);
+                if (kPair) umma_f16_pair(d, ad + 2u * k, bd + 128u * k, idesc, add | k);
+                else umma_f16(d, ad + 2u * k, bd + 128u * k, idesc, add | k);
               }
             }
           } else {
@@ -624,7 +643,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
       if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, p.dev_status, 300)) break;
       __syncwarp();
       tc_fence_after_sync();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN;
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * acc_cols;
+      // the further accumulators of a chunk whose first one has been loaded into v
+      auto add_sets = [&](int c, uint32_t (&v)[32]) {
+        for (int i = 1; kTwo && i <= main_sets; ++i) {
+          uint32_t w[32];
+          tmem_ld_32x32(t_row + (i == main_sets ? sets - 1 : i) * BN + c * 32, w);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+        }
+      };
       if constexpr (!kSplit) {
         // One chunk at a time per warp (measured: several accumulator loads in flight per warp do not
         // shorten the epilogue; a second warp on the same scheduler does).
@@ -634,6 +663,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
           tmem_ld_32x32(t_row + c * 32, v);
           if (c + kEpiSub < chunks) load_residual(p, out_row, n0 + (c + kEpiSub) * 32, res_next);
           tmem_ld_wait();
+          add_sets(c, v);
           const int nb = n0 + c * 32;
           if (!kConv && p.ragged) {
             float f[32];
@@ -665,6 +695,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
             uint32_t v[32];
             tmem_ld_32x32(t_row + c * 32, v);
             tmem_ld_wait();
+            add_sets(c, v);
             const uint32_t owner = c / cps;
             const uint32_t slot = (crank < owner) ? crank : crank - 1;   // this CTA's slot at the owner
             const uint32_t base = recv_base + ((slot * cps + (c % cps)) * 8u * kBM + row_in_tile) * 16u;
@@ -692,6 +723,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
           const int c = crank * cps + cc;
           if (cc + kEpiSub < cps) load_residual(p, out_row, n0 + (c + kEpiSub) * 32, res_next);
           tmem_ld_wait();
+          add_sets(c, v);
           float f[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
@@ -789,6 +821,7 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
     for (int bn = 32; bn <= 256; bn += 32) {
       if (b_kn && (pair ? bn % 128 : bn % 64)) continue;  // MN-major B is loaded in 64-column boxes
       if (force_bn && bn != force_bn) continue;
+      if (2 * acc_sets(parts, bn) * bn > 512) continue;   // tensor memory
       const int units_m = pair ? (tiles_m + 1) / 2 : tiles_m;
       const int tiles = units_m * ((N + bn - 1) / bn);
       for (int split = 1; split <= (pair ? 1 : 4); split *= 2) {
@@ -797,7 +830,7 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
         const int st = stages_for(bn, split, pair, extra_smem, parts);
         if (st < 3) continue;
         const int width = pair ? 2 : split;
-        const int clusters = width > 1 ? resident_clusters(gemm_conv_kernel<false, false, true>, kGemmThreads, kSmemBudget, width, g_clusters) : sms;
+        const int clusters = width > 1 ? resident_clusters(gemm_conv_kernel<false, false, true, false>, kGemmThreads, kSmemBudget, width, g_clusters) : sms;
         const int par = tiles < clusters ? tiles : clusters;
         const int rounds = (tiles + par - 1) / par;
         const double bytes = 16384.0 + bn * (pair ? 64.0 : 128.0);
@@ -818,7 +851,7 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
   return best;
 }
 
-template <bool kConv, bool kPair, bool kSplit>
+template <bool kConv, bool kPair, bool kSplit, bool kTwo>
 static int launch_one(const GemmParams& p, int num_units, cudaStream_t stream) {
   const int b_rows = kPair ? p.bn / 2 : p.bn;
   const int smem = p.stages * p.parts * (kABytes + b_rows * 128) + recv_bytes(p.bn, kSplit ? p.split : 1) + kSmemMisc +
@@ -827,7 +860,7 @@ static int launch_one(const GemmParams& p, int num_units, cudaStream_t stream) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(gemm_conv_kernel<kConv, kPair, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget),
+    if (int rc = check_cuda(cudaFuncSetAttribute(gemm_conv_kernel<kConv, kPair, kSplit, kTwo>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBudget),
                             "cudaFuncSetAttribute(gemm)"))
       return rc;
     configured[dev] = true;
@@ -836,16 +869,16 @@ static int launch_one(const GemmParams& p, int num_units, cudaStream_t stream) {
   int clusters = sm_count() / width;
   if (clusters > num_units) clusters = num_units;
   if (clusters < 1) clusters = 1;
-  return launch_kernel("gemm_conv_kernel launch", gemm_conv_kernel<kConv, kPair, kSplit>, dim3(clusters * width), dim3(kGemmThreads), smem,
+  return launch_kernel("gemm_conv_kernel launch", gemm_conv_kernel<kConv, kPair, kSplit, kTwo>, dim3(clusters * width), dim3(kGemmThreads), smem,
                        stream, width, p);
 }
 
 // tiles_m: 128-row tiles along M; tiles_n: tiles along N
-template <bool kConv>
+template <bool kConv, bool kTwo = false>
 static int launch(const GemmParams& p, int tiles_m, int tiles_n, cudaStream_t stream) {
-  if (p.pair) return launch_one<kConv, true, false>(p, ((tiles_m + 1) / 2) * tiles_n, stream);
-  if (p.split > 1) return launch_one<kConv, false, true>(p, tiles_m * tiles_n, stream);
-  return launch_one<kConv, false, false>(p, tiles_m * tiles_n, stream);
+  if (p.pair) return launch_one<kConv, true, false, kTwo>(p, ((tiles_m + 1) / 2) * tiles_n, stream);
+  if (p.split > 1) return launch_one<kConv, false, true, kTwo>(p, tiles_m * tiles_n, stream);
+  return launch_one<kConv, false, false, kTwo>(p, tiles_m * tiles_n, stream);
 }
 
 static int aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -1238,7 +1271,7 @@ extern "C" int bxl_gemm_split_f32(const float* A, const float* B, float* C, int 
   const TileConfig tc = choose_tiles(tiles_m, N, (K + kBK - 1) / kBK, true, g_force_bn, g_force_split,
                                      g_force_pair < 0 ? kDefaultPair : g_force_pair, 0.0, 0, 2, true);
   const int BN = tc.bn;
-  // C = A_hi*B_hi + A_hi*B_lo + A_lo*B_hi, one fp32 accumulator.  The operand stream bounds the K loop, so a
+  // C = A_hi*B_hi + A_hi*B_lo + A_lo*B_hi.  The operand stream bounds the K loop, so a
   // ring slot holds the four parts of a k-block and three products are formed from it (four tiles copied for
   // three products; one product at a time copied six): 8192 x 640 x 640 42.3 -> 33.8 us, 4096 x 2048 x 2048
   // 98.4 -> 86.6 us, 256 x 512 x 512 14.5 -> 9.4 us, the parts in one launch included.
@@ -1259,7 +1292,7 @@ extern "C" int bxl_gemm_split_f32(const float* A, const float* B, float* C, int 
   p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair;
   p.C = C, p.ldc = N, p.out_f32 = 1;
   p.dev_status = st;
-  return launch<false>(p, tiles_m, (N + BN - 1) / BN, s);
+  return launch<false, true>(p, tiles_m, (N + BN - 1) / BN, s);
 }
 
 // ---- convolution --------------------------------------------------------------------
