@@ -116,7 +116,14 @@ __device__ __forceinline__ void st_global_v8(void* ptr, uint32_t a, uint32_t b, 
                "r"(f), "r"(g), "r"(h)
                : "memory");
 }
-
+// 32-byte load (32-byte aligned): a whole sector per instruction.  Residual rows through it (two loads of a
+// thread's 64 bytes instead of four): linear 2048 x 1280 x 1280 12.2 -> 11.1 us, 8192 x 640 x 640 17.0 -> 15.4 us.
+__device__ __forceinline__ void ld_global_v8(const void* ptr, uint4& lo, uint4& hi) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(lo.x), "=r"(lo.y), "=r"(lo.z), "=r"(lo.w), "=r"(hi.x), "=r"(hi.y), "=r"(hi.z), "=r"(hi.w)
+               : "l"(ptr)
+               : "memory");
+}
 
 // ---- thread-block clusters / distributed shared memory ------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {

@@ -128,8 +128,13 @@ __device__ __forceinline__ void load_residual(const GemmParams& p, long long out
   r.valid = (p.residual != nullptr) && !p.ragged && out_row >= 0 && (nb + 32 <= p.N);
   if (r.valid) {
     const __half* rr = p.residual + out_row * p.ldr + nb;
+    if ((reinterpret_cast<uintptr_t>(rr) & 31u) == 0) {
+      ld_global_v8(rr, r.u[0], r.u[1]);
+      ld_global_v8(rr + 16, r.u[2], r.u[3]);
+    } else {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) r.u[q] = *reinterpret_cast<const uint4*>(rr + q * 8);
+      for (int q = 0; q < 4; ++q) r.u[q] = *reinterpret_cast<const uint4*>(rr + q * 8);
+    }
   }
 }
 
@@ -207,7 +212,13 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, float (&f)[32],
   }
   if (p.out_f32) {
     float* cr = static_cast<float*>(p.C) + out_row * p.ldc + nb;
-    if (fullw) {
+    if (fullw && (reinterpret_cast<uintptr_t>(cr) & 31u) == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        st_global_v8(cr + 8 * q, __float_as_uint(f[8 * q]), __float_as_uint(f[8 * q + 1]), __float_as_uint(f[8 * q + 2]),
+                     __float_as_uint(f[8 * q + 3]), __float_as_uint(f[8 * q + 4]), __float_as_uint(f[8 * q + 5]),
+                     __float_as_uint(f[8 * q + 6]), __float_as_uint(f[8 * q + 7]));
+    } else if (fullw) {
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *reinterpret_cast<float4*>(cr + q * 4) = make_float4(f[q * 4], f[q * 4 + 1], f[q * 4 + 2], f[q * 4 + 3]);
