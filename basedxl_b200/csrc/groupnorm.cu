@@ -242,6 +242,10 @@ struct GnFusedParams {
   int W;
 };
 
+// kDepth: pixels a thread loads before it uses the first.  8 where one CTA has an SM and a thread has 16 pixels or more,
+// so that what is in flight covers the latency: 2 x 320 x 256 x 256 180 -> 90 us, 2 x 960 x 128 x 128 128 -> 61, 2 x 320 x
+// 128 x 128 37.2 -> 33.6; 4 elsewhere, where deeper loads made the short passes slower (2 x 640 x 64 x 64 17.9 -> 20.8).
+template <int kDepth>
 __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParams p) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) unsigned char gnf_smem[];
@@ -278,16 +282,17 @@ __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParam
   const __half* xb = p.x + (long long)img * p.img_stride + (long long)cblk * cb + (long long)v * 8;
   if (r < rows) {
     int pix = p0 + r;
-    for (; pix + 3 * rows < p1; pix += 4 * rows) {
-      const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
-      const uint4 u1 = __ldg(reinterpret_cast<const uint4*>(xb + (long long)(pix + rows) * p.C));
-      const uint4 u2 = __ldg(reinterpret_cast<const uint4*>(xb + (long long)(pix + 2 * rows) * p.C));
-      const uint4 u3 = __ldg(reinterpret_cast<const uint4*>(xb + (long long)(pix + 3 * rows) * p.C));
-      if (p.keep) {
-        s_slab[(size_t)(pix - p0) * bv + v] = u0, s_slab[(size_t)(pix + rows - p0) * bv + v] = u1;
-        s_slab[(size_t)(pix + 2 * rows - p0) * bv + v] = u2, s_slab[(size_t)(pix + 3 * rows - p0) * bv + v] = u3;
+    // kDepth independent loads in flight per thread: with so few warps on an SM the latency of a load, not the
+    // memory, bounds the pass
+    for (; pix + (kDepth - 1) * rows < p1; pix += kDepth * rows) {
+      uint4 u[kDepth];
+#pragma unroll
+      for (int j = 0; j < kDepth; ++j) u[j] = __ldg(reinterpret_cast<const uint4*>(xb + (long long)(pix + j * rows) * p.C));
+#pragma unroll
+      for (int j = 0; j < kDepth; ++j) {
+        if (p.keep) s_slab[(size_t)(pix + j * rows - p0) * bv + v] = u[j];
+        accumulate8(u[j], s1, s2);
       }
-      accumulate8(u0, s1, s2), accumulate8(u1, s1, s2), accumulate8(u2, s1, s2), accumulate8(u3, s1, s2);
     }
     for (; pix < p1; pix += rows) {
       const uint4 u = __ldg(reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
@@ -376,8 +381,7 @@ __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParam
   for (int j = 0; j < 8; ++j) a[j] = s_ab[v * 8 + j], b[j] = s_ab[cb + v * 8 + j];
   __half* yb = p.y + (long long)img * p.img_stride + (long long)cblk * cb + (long long)v * 8;
   const int last_row0 = p.HW - p.W;
-  for (int pix = p0 + r; pix < p1; pix += rows) {
-    const uint4 u = p.keep ? s_slab[(size_t)(pix - p0) * bv + v] : *reinterpret_cast<const uint4*>(xb + (long long)pix * p.C);
+  auto normalise = [&](int pix, const uint4 u) {
     const __half2* h = reinterpret_cast<const __half2*>(&u);
     uint4 o;
     __half2* oh = reinterpret_cast<__half2*>(&o);
@@ -398,6 +402,28 @@ __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParam
         *reinterpret_cast<uint4*>(p.halo_out + ((long long)img * p.W + pix) * p.C + (long long)cblk * cb + v * 8) = o;
       if (pix >= last_row0)
         *reinterpret_cast<uint4*>(p.halo_out + (((long long)p.B + img) * p.W + (pix - last_row0)) * p.C + (long long)cblk * cb + v * 8) = o;
+    }
+  };
+  if (kDepth <= 4) {
+    for (int pix = p0 + r; pix < p1; pix += rows)
+      normalise(pix, p.keep ? s_slab[(size_t)(pix - p0) * bv + v] : *reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
+  } else if (p.keep) {
+#pragma unroll 2
+    for (int pix = p0 + r; pix < p1; pix += rows) normalise(pix, s_slab[(size_t)(pix - p0) * bv + v]);
+  } else {
+    // from the end of the slab, which the first pass has read last: more of it is still in L2
+    int n = (p1 - p0 - r + rows - 1) / rows;   // this thread's pixels (none if not positive)
+    for (; n >= kDepth; n -= kDepth) {
+      const int last = p0 + r + (n - 1) * rows;
+      uint4 u[kDepth];
+#pragma unroll
+      for (int j = 0; j < kDepth; ++j) u[j] = *reinterpret_cast<const uint4*>(xb + (long long)(last - j * rows) * p.C);
+#pragma unroll
+      for (int j = 0; j < kDepth; ++j) normalise(last - j * rows, u[j]);
+    }
+    for (; n > 0; --n) {
+      const int pix = p0 + r + (n - 1) * rows;
+      normalise(pix, *reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
     }
   }
 }
@@ -531,9 +557,10 @@ extern "C" int bxl_groupnorm_fused_f16(const void* x, void* y, long long img_str
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(groupnorm_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024),
-                            "cudaFuncSetAttribute(groupnorm_fused)"))
-      return rc;
+    for (auto kernel : {groupnorm_fused_kernel<4>, groupnorm_fused_kernel<8>})
+      if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024),
+                              "cudaFuncSetAttribute(groupnorm_fused)"))
+        return rc;
     configured[dev] = true;
   }
   p.x = static_cast<const __half*>(x), p.y = static_cast<__half*>(y), p.img_stride = img_stride;
@@ -541,7 +568,8 @@ extern "C" int bxl_groupnorm_fused_f16(const void* x, void* y, long long img_str
   p.fresh_out = fresh_out, p.n_peers = mode == 2 ? n_peers : 0, p.own = own, p.mode = mode, p.eps = eps;
   p.gamma = static_cast<const __half*>(gamma), p.beta = static_cast<const __half*>(beta), p.silu = silu;
   p.halo_out = static_cast<__half*>(halo_out), p.W = W;
-  return launch_kernel("groupnorm_fused_kernel launch", groupnorm_fused_kernel, dim3(cs * nblk, B), dim3(threads), smem,
+  auto kernel = (long long)cs * nblk * B <= sm_count() && per * bv >= 16 * threads ? groupnorm_fused_kernel<8> : groupnorm_fused_kernel<4>;
+  return launch_kernel("groupnorm_fused_kernel launch", kernel, dim3(cs * nblk, B), dim3(threads), smem,
                        (cudaStream_t)stream, cs, p);
 }
 
