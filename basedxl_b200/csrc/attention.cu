@@ -798,11 +798,13 @@ extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long
   static const double kTileCost[kGroups + 1] = {0.0, 0.58, 0.85, 1.0};
   int split = 1, groups = kGroups;
   double best = 1e30;
+  int at_once[5] = {0, sm_count(), 0, 0, 0};
+  for (int w = 2; w <= 4; w *= 2) at_once[w] = resident_clusters(attention_kernel, kAttnThreads, AttnSmem::kTotal, w, g_attn_clusters);
   for (int g = kGroups; g >= 1; --g) {
     const int work = ((q_tiles + g - 1) / g) * heads * B;
     for (int s2 = 1; s2 <= 4; s2 *= 2) {
       if (s2 > total_tiles || (g_force_attn_split && s2 != g_force_attn_split)) continue;
-      const int clusters = s2 > 1 ? resident_clusters(attention_kernel, kAttnThreads, AttnSmem::kTotal, s2, g_attn_clusters) : sm_count();
+      const int clusters = at_once[s2];
       const int rounds = (work + clusters - 1) / clusters;
       const double tc = kTileCost[g < q_tiles ? g : (q_tiles < kGroups ? q_tiles : kGroups)];
       const double cost = (s2 == 1) ? rounds * (total_tiles * tc + 1.5) : rounds * (((total_tiles + s2 - 1) / s2) * tc + 6.5);

@@ -826,6 +826,8 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
                                int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0, int parts = 1, bool heavy = false) {
   const int sms = sm_count();
   TileConfig best{128, 1, stages_for(128, 1, 0, extra_smem, parts), 0};
+  int at_once[5] = {0, sms, 0, 0, 0};
+  for (int w = 2; w <= 4; w *= 2) at_once[w] = resident_clusters(gemm_conv_kernel<false, false, true, false>, kGemmThreads, kSmemBudget, w, g_clusters);
   double best_cost = 1e30;
   for (int pair = 0; pair <= 1; ++pair) {
     if (force_pair >= 0 && pair != force_pair) continue;
@@ -841,7 +843,7 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
         const int st = stages_for(bn, split, pair, extra_smem, parts);
         if (st < 3) continue;
         const int width = pair ? 2 : split;
-        const int clusters = width > 1 ? resident_clusters(gemm_conv_kernel<false, false, true, false>, kGemmThreads, kSmemBudget, width, g_clusters) : sms;
+        const int clusters = at_once[width];
         const int par = tiles < clusters ? tiles : clusters;
         const int rounds = (tiles + par - 1) / par;
         const double bytes = 16384.0 + bn * (pair ? 64.0 : 128.0);
