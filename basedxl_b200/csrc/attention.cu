@@ -14,7 +14,11 @@
 //               registers, packs P to fp16 and stores it to TENSOR MEMORY (tcgen05.st), from where the
 //               P V product reads it as its A operand: P never touches shared memory.  The running
 //               maximum m is only raised when the tile maximum exceeds it by more than 8 (a factor of
-//               256, harmless in fp16/fp32); only then O is rescaled in tensor memory
+//               256, harmless in fp16/fp32), and at the second tile by any amount: the largest
+//               probability of the first 128 keys is then exactly 1, not rounded to fp16 (error
+//               against 64 bits 1 to 3 % smaller at 77 to 231 keys of normal scores, 4 to 13 % where the
+//               scores are three times as peaked; 4096 x 77 13.6 -> 14.1 us, 2 x 10 x 4096 x 4096 138.2 ->
+//               138.1).  Only then O is rescaled in tensor memory
 //               (tcgen05.ld / multiply / tcgen05.st) and the row sum in its register.  The
 //               result is exact: O and the row sum always refer to the same m.
 //               These warpgroups raise their register budget (setmaxnreg) at the expense of the last one.
@@ -570,9 +574,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         }
         const float m_new = fmaxf(m_run, m_tile * sc);
         float alpha = 1.f;
+        const bool raise = j == 1 ? m_new > m_run : m_new > m_run + kRaise;
         if (j == 0) {
           m_run = m_new;  // O and L start from zero: nothing to rescale
-        } else if (m_new > m_run + kRaise) {
+        } else if (raise) {
           alpha = fast_exp2(m_run - m_new);
           m_run = m_new;
         }

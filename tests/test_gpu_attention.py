@@ -221,3 +221,29 @@ def test_attention_keeps_nan_and_infinite_scores():
         assert torch.isnan(y[..., :64]).all(), (value, token)
         assert torch.equal(y[..., 64:], clean[..., 64:])
     _lib.device_status()
+
+
+@pytest.mark.parametrize("L", [64, 77, 100, 128, 154, 231])
+def test_attention_error_with_peaked_scores(L):
+    """The rounding of P to fp16 is relative to the maximum of the first 128 keys (raised only beyond 2^8), so that the
+    dominant probability is exact.  Bound: the error of that arithmetic, restated in 64 bits with P and the result in
+    fp16 and everything else exact, and 2 % for what the restatement leaves out (fp32 sums, scores at 2^-24)."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    heads, Lq = 20, 300
+    gen = torch.Generator().manual_seed(L)
+    q = h16(3 * torch.randn(1, Lq, heads * 64, generator=gen))
+    kv = h16(torch.randn(1, L, 2 * heads * 64, generator=gen))
+    y = ops.attention(q.half().to(dev), [kv.half().to(dev)], heads).cpu().double()
+    _lib.device_status()
+    split = lambda t: t.double().view(-1, heads, 64).transpose(0, 1)
+    k, v = kv[0].chunk(2, dim=1)
+    s = split(q[0]) @ split(k).transpose(1, 2) / 8 * 1.4426950408889634
+    exact = torch.softmax(s * 0.6931471805599453, -1) @ split(v)
+    m = s[..., :128].amax(-1, keepdim=True)
+    top = s.amax(-1, keepdim=True)
+    p = torch.exp2(s - torch.where(top > m + 8, top, m))
+    model = ((p.half().double() @ split(v)) / p.sum(-1, keepdim=True)).half().double()
+    err = lambda o: float((o - exact).norm() / exact.norm())
+    got = err(split(y[0]))
+    assert got <= 1.02 * err(model), f"{got:.4e} > 1.02 * {err(model):.4e}"
