@@ -582,12 +582,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
           m_run = m_new;
         }
         const bool rescale = __any_sync(0xffffffffu, alpha != 1.f);
+        // as long as every score is -inf: P = 2^(-inf - 0) = 0, and the first finite maximum is raised to
+        const float m_ref = m_run == -INFINITY ? 0.f : m_run;
         // P = exp2(S*scale - m) in fp32, summed in fp32, packed to fp16 for the tensor core:
         // two per 32-bit word
         uint32_t pa[32];
         float sum0, sum1;
         if (valid == kTileKV) {
-          const f32x2 sc2 = pair2(sc, sc), nm2 = pair2(-m_run, -m_run);
+          const f32x2 sc2 = pair2(sc, sc), nm2 = pair2(-m_ref, -m_ref);
           f32x2 q0 = pair2(0.f, 0.f), q1 = q0;
           // spread evenly over the row, so that both units stay busy
           auto on_fma = [](int k) { return (k * kPolyOf16) / 16 != ((k + 1) * kPolyOf16) / 16; };
@@ -601,8 +603,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
           unpair2(q1, u0, u1), sum1 = u0 + u1;
         } else {
           // ragged last tile of a slot: columns >= valid contribute nothing
-          sum0 = ragged_chunk_p<0>(v0, pa, valid, sc, m_run);
-          sum1 = ragged_chunk_p<16>(v1, pa, valid - 32, sc, m_run);
+          sum0 = ragged_chunk_p<0>(v0, pa, valid, sc, m_ref);
+          sum1 = ragged_chunk_p<16>(v1, pa, valid - 32, sc, m_ref);
         }
         l_run = fmaf(l_run, alpha, sum0 + sum1);
         // the previous P V product of this group must have finished: it read the P buffer, and O
@@ -640,7 +642,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         mbar_arrive(p_full(g));
       }
       if (!ok) break;
-      pend_w = w, pend_l = l_run, pend_m = m_run;
+      // a row without a finite score has the sum 0 (0 / 0 = NaN), not what poly_exp2 makes of -inf
+      pend_w = w, pend_l = m_run == -INFINITY ? 0.f * l_run : l_run, pend_m = m_run;
     }
     if (ok && pend_w >= 0) {
       if (S == 1) {

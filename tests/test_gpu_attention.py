@@ -247,3 +247,27 @@ def test_attention_error_with_peaked_scores(L):
     err = lambda o: float((o - exact).norm() / exact.norm())
     got = err(split(y[0]))
     assert got <= 1.02 * err(model), f"{got:.4e} > 1.02 * {err(model):.4e}"
+
+
+@pytest.mark.parametrize("split", [0, 1, 2, 4])
+@pytest.mark.parametrize("masked", [1, 63, 64, 65, 128, 129, 200, 319, 320])
+def test_attention_after_keys_of_minus_infinity(masked, split):
+    """Keys whose scores are -inf (a mask feature, left padding) weigh nothing, however many come first; a row that has
+    no other key is NaN."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    gen = torch.Generator().manual_seed(masked)
+    q, kv = h16(torch.randn(1, 200, 128, generator=gen)), h16(torch.randn(1, 320, 256, generator=gen))
+    q[..., 5] = q[..., 70] = 1.0
+    kv[0, :masked, 5] = kv[0, :masked, 70] = float("-inf")
+    l = _lib.lib()
+    _lib.check(l.bxl_debug_force_attn_split(split), l, kernels=0)
+    try:
+        y = ops.attention(q.half().to(dev), [kv.half().to(dev)], 2)
+        _lib.device_status()
+    finally:
+        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
+    if masked == 320:
+        assert torch.isnan(y).all()
+    else:
+        assert_close(y, po._sdpa_heads(q, kv[:, masked:], 2), what=f"{masked} keys of -inf first, split {split}")
