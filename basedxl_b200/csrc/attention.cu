@@ -184,9 +184,16 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
       "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Ragged last tile of a slot, one 32-column chunk with nv valid columns (warp-uniform): row
-// maximum, and P = exp2(s*sc - m) packed into pk[kOff .. kOff+15] with its sum.  Chunks without
+// maximum, and P = exp2(s*sc - m) packed into pk[off .. off+15] with its sum.  Chunks without
 // a valid column cost nothing.
 __device__ __forceinline__ float ragged_chunk_max(const uint32_t (&v)[32], int nv) {
   float m = -INFINITY;
@@ -205,15 +212,15 @@ __device__ __forceinline__ float ragged_chunk_max(const uint32_t (&v)[32], int n
   }
   return m;
 }
-template <int kOff>
-__device__ __forceinline__ float ragged_chunk_p(const uint32_t (&v)[32], uint32_t (&pk)[32], int nv, float sc, float m) {
+template <int kWords>
+__device__ __forceinline__ float ragged_chunk_p(const uint32_t (&v)[32], uint32_t (&pk)[kWords], int off, int nv, float sc, float m) {
   float s0 = 0.f, s1 = 0.f;
   if (nv >= 32) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const float a = fast_exp2(fmaf(__uint_as_float(v[2 * i]), sc, -m)), b = fast_exp2(fmaf(__uint_as_float(v[2 * i + 1]), sc, -m));
       s0 += a, s1 += b;
-      pk[kOff + i] = pack_f16x2(a, b);
+      pk[off + i] = pack_f16x2(a, b);
     }
   } else if (nv > 0) {
 #pragma unroll
@@ -221,19 +228,18 @@ __device__ __forceinline__ float ragged_chunk_p(const uint32_t (&v)[32], uint32_
       const float a = (2 * i < nv) ? fast_exp2(fmaf(__uint_as_float(v[2 * i]), sc, -m)) : 0.f;
       const float b = (2 * i + 1 < nv) ? fast_exp2(fmaf(__uint_as_float(v[2 * i + 1]), sc, -m)) : 0.f;
       s0 += a, s1 += b;
-      pk[kOff + i] = pack_f16x2(a, b);
+      pk[off + i] = pack_f16x2(a, b);
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) pk[kOff + i] = 0u;
+    for (int i = 0; i < 16; ++i) pk[off + i] = 0u;
   }
   return s0 + s1;
 }
 
 // One query row of a finished unit: read O (64 fp32 columns of this thread's TMEM lane),
-// normalise by the row sum and store 64 halves.  Kept out of line: it is called from inside the
-// K/V loop, where the registers are needed for the row of S.
-__device__ __noinline__ void attn_store_row(uint32_t o_addr, __half* dst, float inv_l) {
+// normalise by the row sum and store 64 halves.
+__device__ __forceinline__ void attn_store_row_inline(uint32_t o_addr, __half* dst, float inv_l) {
   uint32_t o0[32], o1[32];
   tmem_ld_32x32(o_addr, o0);
   tmem_ld_32x32(o_addr + 32, o1);
@@ -256,6 +262,11 @@ __device__ __noinline__ void attn_store_row(uint32_t o_addr, __half* dst, float 
     for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
   }
 }
+
+// Out of line for attention_kernel, which calls it inside its K/V loop, where the registers are needed for the
+// row of S.  No other kernel calls this copy: a function that kernels of different register counts share is
+// compiled for one of them.
+__device__ __noinline__ void attn_store_row(uint32_t o_addr, __half* dst, float inv_l) { attn_store_row_inline(o_addr, dst, inv_l); }
 
 __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -603,8 +614,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
           unpair2(q1, u0, u1), sum1 = u0 + u1;
         } else {
           // ragged last tile of a slot: columns >= valid contribute nothing
-          sum0 = ragged_chunk_p<0>(v0, pa, valid, sc, m_ref);
-          sum1 = ragged_chunk_p<16>(v1, pa, valid - 32, sc, m_ref);
+          sum0 = ragged_chunk_p(v0, pa, 0, valid, sc, m_ref);
+          sum1 = ragged_chunk_p(v1, pa, 16, valid - 32, sc, m_ref);
         }
         l_run = fmaf(l_run, alpha, sum0 + sum1);
         // the previous P V product of this group must have finished: it read the P buffer, and O
@@ -738,8 +749,160 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
   }
 }
 
+// Few keys (one slot of at most 128 tokens: cross-attention with the text).  What bounds such a call is latency:
+// load, Q K^T, softmax, P V and store of a query tile follow one another.  So a CTA serves ONE query tile of one
+// (image, head), and four CTAs on an SM overlap instead of a pipeline inside one.  The scores of all keys are in
+// tensor memory at one time: the exact row maximum is the reference of the exponentials, nothing is rescaled, and
+// the keys are read in one pass (in 64-token tiles 77 keys took two).  Measured (attention_kernel -> this one):
+// 2 x 10 heads, 77 keys: 1024 queries 7.3 -> 6.4 us, 4096 13.6 -> 10.8 (21 MB: 2.0 TB/s), 16384 30.5 -> 27.0;
+// 64 queries of 5 heads 4.9 -> 3.4.  The same with 256 columns and two CTAs per SM was slower than
+// attention_kernel at 154 keys (16.1 -> 16.8) and 231 (19.0 -> 20.2).
+//   warps 0..3  softmax: thread r owns query row r (= TMEM lane r); the row is read twice, 32 columns at a time
+//   warp 4      TMA, tcgen05.mma and tensor memory
+// Tensor memory, 128 columns: S [0, keys), P (two fp16 per column) over the columns of S that have been read,
+// O in [64, 128) over the rest of S, written once every thread has read its row.  Shared memory is asked for in
+// the proportion that these columns are of the SM's 512: CTAs that fit beside one another (of this kernel, or of
+// the launch after it, which may start early) then never wait for tensor memory.
+constexpr int kShortThreads = 160;
+constexpr int kShortKeys = 128;
+struct ShortSmem {
+  static constexpr int kQ = 0, kK = kQBytes, kV = kK + kShortKeys * kHeadDim * 2, kBar = kV + kShortKeys * kHeadDim * 2;
+  static constexpr int kTotal = (228 * kShortKeys / 512 - 1) * 1024;   // and 1 KB that the system takes
+  static_assert(kBar + 64 + 1024 <= kTotal, "shared memory");
+};
+
+__global__ void __launch_bounds__(kShortThreads, 512 / kShortKeys) attention_short_kernel(const __grid_constant__ AttnParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t qk_full = smem_base + ShortSmem::kBar, v_full = qk_full + 8, s_full = qk_full + 16, p_full = qk_full + 24, o_full = qk_full + 32;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + ShortSmem::kBar + 48);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + ShortSmem::kBar + 56);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(qk_full, 1);
+    mbar_init(v_full, 1);
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 128);
+    mbar_init(o_full, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 4) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), kShortKeys);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();  // not before: the next launch's CTAs must not take tensor memory that this grid still waits for
+  pdl_wait();  // the set-up above overlaps the previous kernel's tail; global data from here on
+
+  const int q_tiles = (p.L_q + kTileQ - 1) / kTileQ;
+  const int q_row0 = static_cast<int>(blockIdx.x % q_tiles) * kTileQ;
+  const int head = static_cast<int>(blockIdx.x / q_tiles) % p.heads, img = static_cast<int>(blockIdx.x / q_tiles) / p.heads;
+  const int keys = p.L_slot;
+  const int keys16 = (keys + 15) & ~15;   // rows of the K and V boxes; those past the last key arrive as zeros
+  if (warp == 4) {
+    const bool leader = elect_one();
+    if (leader) {
+      mbar_arrive_expect_tx(qk_full, static_cast<uint32_t>(kQBytes + keys16 * kHeadDim * 2));
+      tma_load_3d(smem_base + ShortSmem::kQ, &p.q_map, qk_full, head * kHeadDim, q_row0, img);
+      tma_load_3d(smem_base + ShortSmem::kK, &p.kv_map[0], qk_full, head * kHeadDim, 0, img);
+      mbar_arrive_expect_tx(v_full, static_cast<uint32_t>(keys16 * kHeadDim * 2));
+      tma_load_3d(smem_base + ShortSmem::kV, &p.kv_map[0], v_full, p.v_col0 + head * kHeadDim, 0, img);
+    }
+    __syncwarp();
+    if (mbar_wait_warp(qk_full, 0, abort_flag, p.dev_status, 700)) {
+      tc_fence_after_sync();
+      const uint64_t qdesc = make_smem_desc_sw128(smem_base + ShortSmem::kQ, 16, 1024), kdesc = make_smem_desc_sw128(smem_base + ShortSmem::kK, 16, 1024);
+      const uint32_t idesc = make_idesc_f16(kTileQ, keys16, 0, 0);   // S = Q K^T, both K-major
+      if (leader) {
+#pragma unroll
+        for (int k = 0; k < kHeadDim / 16; ++k) umma_f16(tmem_base, qdesc + 2u * k, kdesc + 2u * k, idesc, k != 0);
+        umma_commit(s_full);
+      }
+      __syncwarp();
+      if (mbar_wait_warp(v_full, 0, abort_flag, p.dev_status, 701) && mbar_wait_warp(p_full, 0, abort_flag, p.dev_status, 702)) {
+        tc_fence_after_sync();
+        const uint64_t vdesc = make_smem_desc_sw128(smem_base + ShortSmem::kV, 16, 1024);
+        const uint32_t idesc_o = make_idesc_f16(kTileQ, kHeadDim, 0, 1);  // O = P V, V MN-major
+        if (leader) {
+          for (int k = 0; k < keys16 / 16; ++k)
+            umma_f16_ts(tmem_base + kShortKeys / 2, tmem_base + 8u * k, vdesc + 128u * k, idesc_o, k != 0);
+          umma_commit(o_full);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    const int row = warp * 32 + lane;
+    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+    const float sc = p.scale_log2e;
+    if (mbar_wait(s_full, 0, abort_flag, p.dev_status, 710)) {
+      __syncwarp();
+      tc_fence_after_sync();
+      float m = -INFINITY;
+      uint32_t v[32];
+      for (int c = 0; c < keys; c += 32) {
+        tmem_ld_32x32(t_lane + c, v);
+        tmem_ld_wait();
+        m = fmaxf(m, ragged_chunk_max(v, keys - c));
+      }
+      m *= sc;
+      float l = 0.f;
+      for (int c = 0; c < keys; c += 32) {
+        tmem_ld_32x32(t_lane + c, v);
+        tmem_ld_wait();
+        uint32_t pk[16];
+        l += ragged_chunk_p(v, pk, 0, keys - c, sc, m);
+        tmem_st_32x16(t_lane + c / 2, pk);   // over columns of S that this thread has read
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      mbar_arrive(p_full);
+      if (mbar_wait(o_full, 0, abort_flag, p.dev_status, 711)) {
+        __syncwarp();
+        tc_fence_after_sync();
+        __half* dst = q_row0 + row < p.L_q ? p.out + (long long)img * p.out_img_stride + (long long)(q_row0 + row) * p.ld_out + head * kHeadDim : nullptr;
+        attn_store_row_inline(t_lane + kShortKeys / 2, dst, 1.f / l);
+      }
+    }
+  }
+  // ---- teardown ---------------------------------------------------------------
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {
+    const unsigned long long t0 = global_timer_ns();
+    while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 4) {
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, kShortKeys);
+  }
+}
+
 static int g_attn_clusters[64][5] = {};
 static int g_force_attn_split = 0;  // test hook: 0 = choose
+
+static int launch_short(const AttnParams& p, cudaStream_t stream) {
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(attention_short_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ShortSmem::kTotal),
+                            "cudaFuncSetAttribute(attention_short)"))
+      return rc;
+    configured[dev] = true;
+  }
+  const int q_tiles = (p.L_q + kTileQ - 1) / kTileQ;
+  return launch_kernel("attention_short_kernel launch", attention_short_kernel, dim3(q_tiles * p.heads * p.B), dim3(kShortThreads),
+                       ShortSmem::kTotal, stream, 1, p);
+}
 
 }  // namespace bxl
 
@@ -774,12 +937,14 @@ extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long
     uint32_t box[3] = {kHeadDim, kTileQ, 1};
     if (int rc = encode_tmap_f16(&p.q_map, q, 3, dims, str, box)) return rc;
   }
-  for (int s = 0; s < kMaxSlots; ++s) {
+  // attention_short_kernel is the faster one at every measured size that it serves; a forced K/V split means the other
+  const bool few_keys = n_slots == 1 && L_slot <= kShortKeys && !g_force_attn_split;
+  for (int s = 0; s < (few_keys ? 1 : kMaxSlots); ++s) {
     const void* base = kv_slots[s < n_slots ? s : 0];
     if (!base) return fail(kErrInvalidArg, "bxl_attn_fwd_f16: slot %d null", s);
     uint64_t dims[3] = {(uint64_t)(v_col0 + heads * kHeadDim), (uint64_t)L_slot, (uint64_t)B};
     uint64_t str[2] = {(uint64_t)ld_kv * 2, (uint64_t)kv_img_stride * 2};
-    uint32_t box[3] = {kHeadDim, kTileKV, 1};
+    uint32_t box[3] = {kHeadDim, (uint32_t)(few_keys ? (L_slot + 15) / 16 * 16 : kTileKV), 1};
     if (int rc = encode_tmap_f16(&p.kv_map[s], base, 3, dims, str, box)) return rc;
   }
   p.n_slots = n_slots, p.L_q = L_q, p.L_slot = L_slot, p.heads = heads, p.B = B, p.v_col0 = v_col0;
@@ -787,6 +952,7 @@ extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long
   p.out_img_stride = out_img_stride, p.ld_out = ld_out;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.dev_status = st;
+  if (few_keys) return launch_short(p, (cudaStream_t)stream);
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);

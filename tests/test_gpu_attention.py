@@ -271,3 +271,22 @@ def test_attention_after_keys_of_minus_infinity(masked, split):
         assert torch.isnan(y).all()
     else:
         assert_close(y, po._sdpa_heads(q, kv[:, masked:], 2), what=f"{masked} keys of -inf first, split {split}")
+
+
+@pytest.mark.parametrize("keys", [1, 15, 16, 17, 32, 33, 64, 65, 77, 112, 127, 128, 129])
+@pytest.mark.parametrize("Lq,offset", [(1, 0), (128, 8), (129, 0), (300, 8)])
+def test_attention_with_few_keys(keys, Lq, offset):
+    """One slot of up to 128 keys in one pass, up to the first length that takes the general kernel: keys on, before and
+    after a 16- and a 32-column boundary, ragged query tiles, output rows at 32-byte boundaries and between them."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    B, heads = 2, 3
+    C = heads * 64
+    gen = torch.Generator().manual_seed(keys + 1000 * Lq)
+    q, kv = h16(torch.randn(B, Lq, C, generator=gen)), h16(torch.randn(B, keys, 2 * C, generator=gen))
+    store = torch.full((B, Lq, C + 16), 7.0, dtype=torch.float16, device=dev)
+    out = store[..., offset : offset + C]
+    ops.attention(q.half().to(dev), [kv.half().to(dev)], heads, out=out)
+    _lib.device_status()
+    assert_close(out, po._sdpa_heads(q, kv, heads), what=f"attention of {keys} keys, Lq {Lq}")
+    assert bool((store[..., :offset] == 7).all()) and bool((store[..., offset + C :] == 7).all())
