@@ -3,43 +3,41 @@
 // slots [B, L_slot, 2C] (K in columns [0,C), V in [C,2C), head h at columns
 // h*64..h*64+63).  The slots are read IN PLACE through one TMA descriptor per
 // slot: the own strip's fresh K/V and the peers' stale K/V are never
-// concatenated.  The same kernel serves cross-attention (one slot, 77 tokens).
+// concatenated.  attention_short_kernel serves one slot of few keys (cross-attention).
 //
-// Work unit = up to 384 queries (three tiles of 128) of one (image, head).  A CTA walks several units
-// (or, with a K/V split, a cluster of 2 or 4 CTAs shares one unit).  512 threads:
-//   warps 0..11 three softmax groups of four warps: thread r of a group owns query row r of its
-//               tile (= TMEM lane r).  Per K/V tile (64 tokens) it reads its row of S once, releases S at
-//               once so the next Q K^T can start, takes the row maximum, forms P = exp2(S*scale - m) in
-//               fp32 (14 of 16 on the special-function unit, 2 on the FMA pipe), sums the row in fp32
-//               registers, packs P to fp16 and stores it to TENSOR MEMORY (tcgen05.st), from where the
-//               P V product reads it as its A operand: P never touches shared memory.  The running
-//               maximum m is only raised when the tile maximum exceeds it by more than 8 (a factor of
-//               256, harmless in fp16/fp32), and at the second tile by any amount: the largest
-//               probability of the first 128 keys is then exactly 1, not rounded to fp16 (error
-//               against 64 bits 1 to 3 % smaller at 77 to 231 keys of normal scores, 4 to 13 % where the
-//               scores are three times as peaked; 4096 x 77 13.6 -> 14.1 us, 2 x 10 x 4096 x 4096 138.2 ->
-//               138.1).  Only then O is rescaled in tensor memory
-//               (tcgen05.ld / multiply / tcgen05.st) and the row sum in its register.  The
-//               result is exact: O and the row sum always refer to the same m.
-//               These warpgroups raise their register budget (setmaxnreg) at the expense of the last one.
-//   warp 12     TMA producer: the Q tiles of a unit (double buffered across units), then a
-//               ring of {K tile, V tile} (64 tokens x 64) shared by the query tiles
-//   warps 13..15 tcgen05.mma issuers, one per query tile; warp 13 owns tensor memory
+// Work unit of attention_kernel<kGroups, kTileKV> = up to kGroups query tiles of 128 rows of one (image, head):
+// three with key tiles of 64 tokens, or two with 128.  A CTA walks several units (or, with a K/V split, a cluster
+// of 2 or 4 CTAs shares one unit).  Warps:
+//   4 per group softmax: thread r of a group owns query row r of its tile (= TMEM lane r).  Per K/V tile
+//               it reads its row of S once, releases S at once so the next Q K^T can start, takes the row
+//               maximum, forms P = exp2(S*scale - m) in fp32 (14 of 16 on the special-function unit, 2 on
+//               the FMA pipe), sums the row in fp32 registers, packs P to fp16 and stores it to TENSOR
+//               MEMORY (tcgen05.st), from where the P V product reads it as its A operand: P never touches
+//               shared memory.  The running maximum m is only raised when the tile maximum exceeds it by
+//               more than 8 (a factor of 256, harmless in fp16/fp32) and, while fewer than 128 keys have
+//               been seen, by any amount: the largest probability of the first 128 keys is then exactly 1,
+//               not rounded to fp16 (error against 64 bits 1 to 3 % smaller at 77 to 231 keys of normal
+//               scores, 4 to 13 % where the scores are three times as peaked; 2 x 10 x 4096 x 4096
+//               138.2 -> 138.1 us).  Only then O is rescaled in tensor memory (tcgen05.ld / multiply /
+//               tcgen05.st) and the row sum in its register.  The result is exact: O and the row sum always
+//               refer to the same m.
+//               These warps raise their register budget (setmaxnreg) at the expense of the others.
+//   1 TMA producer: the Q tiles of a unit (double buffered across units), then a ring of {K tile, V tile}
+//               shared by the query tiles
+//   kGroups tcgen05.mma issuers, one per query tile; the first owns tensor memory
 //
 // While one group runs its softmax the tensor core works for the others; the K/V tiles of
 // all units of a CTA form one stream, so the first Q K^T of the next unit and the read-out of
 // the finished unit's output overlap the unit boundary.
 //
 // Roofline: tensor cores; algorithmic FLOPs = 4 * L_q * L_kv * 64 per (image, head).  With head dimension 64
-// the exponentials (16 per clock and SM) are the narrowest resource, 1150 TFLOP/s at 1.9 GHz.  Counters at
-// 2 x 20 x 4096 x 4096: special-function unit 64 % busy, issue slots 54 %, tensor pipe 36 %: a softmax warp's
-// own dependences (read S, maximum, exponentials, publish P) bound it, so three warps per scheduler work
-// side by side where there were two with tiles of 128 tokens, and 384-query units leave fewer idle SMs in
-// the last round.  Measured (two groups of 128 x 128 tiles -> three of 128 x 64): 2 x 10 x 4096 x 4096
-// 167.8 -> 138.3 us, 2 x 20 x 4096 x 4096 257 -> 232 (741 TFLOP/s), 2 x 10 x 16384 x 16384 1886 -> 1851,
-// 2 x 20 x 1024 x 1024 29.3 -> 25.4, 1024 queries against 4 x 1024 keys 58.4 -> 46.5; 4096 queries against 77 keys
-// 13.3 -> 13.6, 16384 against 77 37.1 -> 30.5.  Exponentials on the FMA pipe: none 144.0 / 243 / 1880 us on the
-// first three shapes, 4 of 16 137.8 / 242 / 1878.
+// the exponentials are the narrowest resource: 14 of 16 scores at 16 per clock and SM, 1315 TFLOP/s at 1.9 GHz.
+// A softmax warp's own dependences (read S, maximum, exponentials, publish P) bound the kernel: 64 % of that unit,
+// 54 % of the issue slots and 36 % of the tensor pipe are busy at 2 x 20 x 4096 x 4096, so three warps per scheduler
+// work side by side where the work fills them.  Measured (two groups of 128-token tiles -> three of 64):
+// 2 x 10 x 4096 x 4096 152 -> 138 us (622 TFLOP/s), 2 x 20 x 4096 x 4096 246 -> 231 (744), 2 x 20 x 1024 x 1024 31.8 -> 25.5,
+// 1024 queries against 4 x 1024 keys 56.9 -> 46.5; at 2 x 10 x 16384 x 16384 the two are the faster (1850 -> 1789).  Exponentials on the FMA pipe: none 144.0 us on the first
+// shape, 4 of 16 137.8.
 
 #include "bxl_common.cuh"
 #include "bxl_host.h"
@@ -47,22 +45,37 @@
 
 namespace bxl {
 
-constexpr int kGroups = 3;                         // softmax warpgroups = query tiles in flight
-constexpr int kWarpLoad = 4 * kGroups;             // producer warp; then one MMA issuer warp per group
-constexpr int kWarpMma = kWarpLoad + 1;
-constexpr int kAttnThreads = (4 * kGroups + 4) * 32;
-constexpr int kSoftmaxRegs = 144;   // registers per thread after the split: 12 x 32 x 144 + 4 x 32 x 80 = 512 x 128
-constexpr int kOtherRegs = 80;
 constexpr int kPolyOf16 = 2;        // score pairs of every 16 whose exponentials run on the FMA pipe
 constexpr int kHeadDim = 64;
 constexpr int kTileQ = 128;
-constexpr int kTileKV = 64;
-constexpr int kKvStages = 6;
-constexpr int kQBytes = kTileQ * kHeadDim * 2, kKvBytes = kTileKV * kHeadDim * 2;   // one Q tile; one K or V tile
-// tensor memory columns: S_g, O_g (fp32), P_g (two fp16 per column, the A operand of the P V product)
-constexpr int kTmemO = kGroups * kTileKV, kTmemP = kTmemO + kGroups * kHeadDim;
-static_assert(kTmemP + kGroups * kTileKV / 2 <= 512, "tensor memory");
+constexpr int kQBytes = kTileQ * kHeadDim * 2;   // one Q tile
 constexpr int kMaxSlots = 8;
+
+// kGroups softmax warpgroups (query tiles in flight), key tiles of kTileKV tokens: <3, 64> or <2, 128>.
+template <int kGroups, int kTileKV>
+struct AttnShape {
+  static constexpr int kWarpLoad = 4 * kGroups;   // producer warp; then one MMA issuer warp per group
+  static constexpr int kWarpMma = kWarpLoad + 1;
+  static constexpr int kThreads = (4 * kGroups + 4) * 32;
+  // registers per thread after the split: 12 x 32 x 144 + 4 x 32 x 80 = 512 x 128; 8 x 32 x 208 + 4 x 32 x 88 = 384 x 168
+  static constexpr int kSoftmaxRegs = kGroups == 3 ? 144 : 208;
+  static constexpr int kOtherRegs = kGroups == 3 ? 80 : 88;
+  static_assert(4 * kGroups * kSoftmaxRegs + 4 * kOtherRegs == (kGroups == 3 ? 16 * 128 : 12 * 168), "the registers of the launch");
+  static constexpr int kKvStages = kTileKV == 64 ? 6 : 4;
+  static constexpr int kKvBytes = kTileKV * kHeadDim * 2;   // one K or V tile
+  // tensor memory columns: S_g, O_g (fp32), P_g (two fp16 per column, the A operand of the P V product)
+  static constexpr int kTmemO = kGroups * kTileKV, kTmemP = kTmemO + kGroups * kHeadDim;
+  static_assert(kTmemP + kGroups * kTileKV / 2 <= 512, "tensor memory");
+  // shared memory: 2 buffers x kGroups Q tiles, the ring of K tiles and that of V tiles, barriers
+  static constexpr int kQ = 0;
+  static constexpr int kK = 2 * kGroups * kQBytes;
+  static constexpr int kV = kK + kKvStages * kKvBytes;
+  static constexpr int kBar = kV + kKvStages * kKvBytes;
+  static constexpr int kTotal = kBar + 1024 + 1024;
+  static_assert(kTotal <= 227 * 1024, "shared memory");
+  // the merge of a K/V split receives 66 values of a half of the rows, or three times those of a quarter, in the ring
+  static_assert(3 * 66 * (kGroups * kTileQ / 4) * 4 <= 2 * kKvStages * kKvBytes, "merge buffer");
+};
 
 struct alignas(64) AttnParams {
   CUtensorMap q_map;               // [C_q cols, L_q, B]
@@ -75,16 +88,8 @@ struct alignas(64) AttnParams {
   long long out_img_stride, ld_out;
   float scale_log2e;               // softmax scale * log2(e)
   int kv_split;                    // K/V range split over a cluster of 1, 2 or 4 CTAs
-  int groups;                      // query tiles per unit (1..kGroups)
+  int groups;                      // query tiles per unit (1..kGroups of the kernel)
   int* dev_status;
-};
-
-struct AttnSmem {
-  static constexpr int kQ = 0;                               // 2 buffers x kGroups tiles
-  static constexpr int kK = 2 * kGroups * kQBytes;
-  static constexpr int kV = kK + kKvStages * kKvBytes;
-  static constexpr int kBar = kV + kKvStages * kKvBytes;
-  static constexpr int kTotal = kBar + 1024 + 1024;
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -264,15 +269,23 @@ __device__ __forceinline__ void attn_store_row_inline(uint32_t o_addr, __half* d
 }
 
 // Out of line for attention_kernel, which calls it inside its K/V loop, where the registers are needed for the
-// row of S.  No other kernel calls this copy: a function that kernels of different register counts share is
-// compiled for one of them.
-__device__ __noinline__ void attn_store_row(uint32_t o_addr, __half* dst, float inv_l) { attn_store_row_inline(o_addr, dst, inv_l); }
+// row of S.  A copy for each kernel: a function that kernels of different register counts share is compiled for
+// one of them.
+template <int kGroups, int kTileKV>
+__device__ __noinline__ void attn_store_row(uint32_t o_addr, __half* dst, float inv_l) {
+  attn_store_row_inline(o_addr, dst, inv_l);
+}
 
-__global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid_constant__ AttnParams p) {
+template <int kGroups, int kTileKV>
+__global__ void __launch_bounds__(AttnShape<kGroups, kTileKV>::kThreads, 1) attention_kernel(const __grid_constant__ AttnParams p) {
+  using Shape = AttnShape<kGroups, kTileKV>;
+  constexpr int kWarpLoad = Shape::kWarpLoad, kWarpMma = Shape::kWarpMma, kKvStages = Shape::kKvStages, kKvBytes = Shape::kKvBytes;
+  constexpr int kTmemO = Shape::kTmemO, kTmemP = Shape::kTmemP;
+  constexpr int kChunks = kTileKV / 32;   // a row of S in registers: chunks of 32 columns
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t bar_base = smem_base + AttnSmem::kBar;
+  const uint32_t bar_base = smem_base + Shape::kBar;
   // barriers: q_full[2], q_empty[2], kv_full[stages], kv_empty[stages], then per group s_full, o_full, p_full, s_free
   auto q_full = [&](int b) { return bar_base + 8u * b; };
   auto q_empty = [&](int b) { return bar_base + 8u * (2 + b); };
@@ -283,8 +296,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
   auto o_full = [&](int g) { return bar_base + 8u * (kGroupBar + kGroups + g); };
   auto p_full = [&](int g) { return bar_base + 8u * (kGroupBar + 2 * kGroups + g); };
   auto s_free = [&](int g) { return bar_base + 8u * (kGroupBar + 3 * kGroups + g); };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + AttnSmem::kBar + 512);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + AttnSmem::kBar + 520);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem_gen + Shape::kBar + 512);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + Shape::kBar + 520);
 
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5;
@@ -345,12 +358,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  // the softmax warps hold a whole row of S (128 values) and of P: give them the registers the
+  // the softmax warps hold a row of S (kTileKV values) and of P: give them the registers the
   // producer / MMA warpgroup does not need
   pdl_wait();  // the set-up above overlaps the previous kernel's tail; global data from here on
 
   if (warp >= kWarpLoad) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape::kOtherRegs));
   if (warp == kWarpLoad) {
     // ======================= TMA producer =======================
     // all 32 lanes run the loop (addresses stay warp-uniform); the elected lane issues
@@ -370,7 +383,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       if (leader) {
         mbar_arrive_expect_tx(q_full(qb), static_cast<uint32_t>(kQBytes) * ng);
         for (int g = 0; g < ng; ++g)
-          tma_load_3d(smem_base + AttnSmem::kQ + (qb * kGroups + g) * kQBytes, &p.q_map, q_full(qb), head * kHeadDim,
+          tma_load_3d(smem_base + Shape::kQ + (qb * kGroups + g) * kQBytes, &p.q_map, q_full(qb), head * kHeadDim,
                       q_row0 + g * kTileQ, img);
       }
       __syncwarp();
@@ -383,8 +396,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         }
         if (leader) {
           mbar_arrive_expect_tx(kv_full(stage), 2 * kKvBytes);
-          tma_load_3d(smem_base + AttnSmem::kK + stage * kKvBytes, &p.kv_map[slot], kv_full(stage), head * kHeadDim, t0, img);
-          tma_load_3d(smem_base + AttnSmem::kV + stage * kKvBytes, &p.kv_map[slot], kv_full(stage),
+          tma_load_3d(smem_base + Shape::kK + stage * kKvBytes, &p.kv_map[slot], kv_full(stage), head * kHeadDim, t0, img);
+          tma_load_3d(smem_base + Shape::kV + stage * kKvBytes, &p.kv_map[slot], kv_full(stage),
                       p.v_col0 + head * kHeadDim, t0, img);
         }
         __syncwarp();
@@ -395,7 +408,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         }
       }
     }
-  } else {
+  } else if (warp < kWarpMma + kGroups) {
     // ======================= MMA issuers =======================
     // One warp per query tile: its waits come true in a fixed order (S copied out, then P published), and
     // a late group holds up nobody.  All 32 lanes run the loop and the waits; the elected lane issues
@@ -418,8 +431,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       if (!mbar_wait_warp(kv_full(stage), phase, abort_flag, p.dev_status, 501)) return false;
       if (n_s > 0 && !mbar_wait_warp(s_free(g), (n_s - 1) & 1u, abort_flag, p.dev_status, 503)) return false;
       tc_fence_after_sync();
-      const uint64_t qdesc = make_smem_desc_sw128(smem_base + AttnSmem::kQ + (qb * kGroups + g) * kQBytes, 16, 1024);
-      const uint64_t kdesc = make_smem_desc_sw128(smem_base + AttnSmem::kK + stage * kKvBytes, 16, 1024);
+      const uint64_t qdesc = make_smem_desc_sw128(smem_base + Shape::kQ + (qb * kGroups + g) * kQBytes, 16, 1024);
+      const uint64_t kdesc = make_smem_desc_sw128(smem_base + Shape::kK + stage * kKvBytes, 16, 1024);
       if (leader) {
 #pragma unroll
         for (int k = 0; k < kHeadDim / 16; ++k) umma_f16(tmem_base + g * kTileKV, qdesc + 2u * k, kdesc + 2u * k, idesc_s, k != 0);
@@ -487,7 +500,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
           // them, so their 16-token steps of the P V product are skipped
           const int k_steps = (min(kTileKV, p.L_slot - ts * kTileKV) + 15) / 16;
           // V tile [64 tokens][64] as stored: MN-major B operand, 8-token groups 1 KB apart
-          const uint64_t vdesc = make_smem_desc_sw128(smem_base + AttnSmem::kV + st * kKvBytes, 16, 1024);
+          const uint64_t vdesc = make_smem_desc_sw128(smem_base + Shape::kV + st * kKvBytes, 16, 1024);
           if (leader) {
 #pragma unroll
             for (int k = 0; k < kTileKV / 16; ++k) {
@@ -517,7 +530,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
     }
   } else {
     // ======================= softmax / output (warps 0..11) =======================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape::kSoftmaxRegs));
     const int g = warp >> 2;               // query tile served by this warp
     const int quarter = warp & 3;          // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;   // query row inside the tile == TMEM lane
@@ -543,7 +556,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       __half* dst = (q_row < p.L_q) ? p.out + (long long)unit_img(pend_w) * p.out_img_stride + (long long)q_row * p.ld_out +
                                           unit_head(pend_w) * kHeadDim
                                     : nullptr;
-      attn_store_row(o_addr, dst, 1.f / pend_l);
+      attn_store_row<kGroups, kTileKV>(o_addr, dst, 1.f / pend_l);
       pend_w = -1;
       return true;
     };
@@ -562,30 +575,35 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         __syncwarp();
         tc_fence_after_sync();
         // the whole row of S into registers, then hand the buffer back
-        uint32_t v0[32], v1[32];
-        tmem_ld_32x32(s_addr, v0);
-        tmem_ld_32x32(s_addr + 32, v1);
+        uint32_t v[kChunks][32];
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(s_addr + 32 * c, v[c]);
         tmem_ld_wait();
         tc_fence_before_sync();
         mbar_arrive(s_free(g));
         // row maximum over the valid columns
         float m_tile;
         if (valid == kTileKV) {
-          float ma = -INFINITY, mb = -INFINITY, mc = -INFINITY, md = -INFINITY;
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            ma = max3(ma, __uint_as_float(v0[i]), __uint_as_float(v0[i + 1]));
-            mb = max3(mb, __uint_as_float(v1[i]), __uint_as_float(v1[i + 1]));
-            mc = max3(mc, __uint_as_float(v0[i + 2]), __uint_as_float(v0[i + 3]));
-            md = max3(md, __uint_as_float(v1[i + 2]), __uint_as_float(v1[i + 3]));
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) {
+              float& m0 = mx[c & 1];
+              float& m1 = mx[2 + (c & 1)];
+              m0 = max3(m0, __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
+              m1 = max3(m1, __uint_as_float(v[c][i + 2]), __uint_as_float(v[c][i + 3]));
+            }
           }
-          m_tile = fmaxf(fmaxf(ma, mb), fmaxf(mc, md));
+          m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
         } else {
-          m_tile = fmaxf(ragged_chunk_max(v0, valid), ragged_chunk_max(v1, valid - 32));
+          m_tile = ragged_chunk_max(v[0], valid);
+#pragma unroll
+          for (int c = 1; c < kChunks; ++c) m_tile = fmaxf(m_tile, ragged_chunk_max(v[c], valid - 32 * c));
         }
         const float m_new = fmaxf(m_run, m_tile * sc);
         float alpha = 1.f;
-        const bool raise = j == 1 ? m_new > m_run : m_new > m_run + kRaise;
+        const bool raise = kTileKV < 128 && j == 1 ? m_new > m_run : m_new > m_run + kRaise;
         if (j == 0) {
           m_run = m_new;  // O and L start from zero: nothing to rescale
         } else if (raise) {
@@ -597,27 +615,32 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
         const float m_ref = m_run == -INFINITY ? 0.f : m_run;
         // P = exp2(S*scale - m) in fp32, summed in fp32, packed to fp16 for the tensor core:
         // two per 32-bit word
-        uint32_t pa[32];
-        float sum0, sum1;
+        uint32_t pa[kTileKV / 2];
+        float sum = 0.f;
         if (valid == kTileKV) {
           const f32x2 sc2 = pair2(sc, sc), nm2 = pair2(-m_ref, -m_ref);
-          f32x2 q0 = pair2(0.f, 0.f), q1 = q0;
+          f32x2 q[2] = {pair2(0.f, 0.f), pair2(0.f, 0.f)};
           // spread evenly over the row, so that both units stay busy
           auto on_fma = [](int k) { return (k * kPolyOf16) / 16 != ((k + 1) * kPolyOf16) / 16; };
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            pa[i] = on_fma(2 * i) ? exp_pair<true>(v0[2 * i], v0[2 * i + 1], sc2, nm2, q0) : exp_pair<false>(v0[2 * i], v0[2 * i + 1], sc2, nm2, q0);
-            pa[16 + i] = on_fma(2 * i + 1) ? exp_pair<true>(v1[2 * i], v1[2 * i + 1], sc2, nm2, q1) : exp_pair<false>(v1[2 * i], v1[2 * i + 1], sc2, nm2, q1);
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c)
+              pa[16 * c + i] = on_fma(kChunks * i + c) ? exp_pair<true>(v[c][2 * i], v[c][2 * i + 1], sc2, nm2, q[c & 1])
+                                                       : exp_pair<false>(v[c][2 * i], v[c][2 * i + 1], sc2, nm2, q[c & 1]);
           }
-          float u0, u1;
-          unpair2(q0, u0, u1), sum0 = u0 + u1;
-          unpair2(q1, u0, u1), sum1 = u0 + u1;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            float u0, u1;
+            unpair2(q[c], u0, u1);
+            sum += u0 + u1;
+          }
         } else {
           // ragged last tile of a slot: columns >= valid contribute nothing
-          sum0 = ragged_chunk_p(v0, pa, 0, valid, sc, m_ref);
-          sum1 = ragged_chunk_p(v1, pa, 16, valid - 32, sc, m_ref);
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c) sum += ragged_chunk_p(v[c], pa, 16 * c, valid - 32 * c, sc, m_ref);
         }
-        l_run = fmaf(l_run, alpha, sum0 + sum1);
+        l_run = fmaf(l_run, alpha, sum);
         // the previous P V product of this group must have finished: it read the P buffer, and O
         // is only touched between two products
         if (j == 0) {
@@ -647,7 +670,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
           }
         }
         // publish P in tensor memory
-        tmem_st_32x32(p_addr, pa);
+#pragma unroll
+        for (int c = 0; c < kChunks / 2; ++c) tmem_st_32x32(p_addr + 32 * c, *reinterpret_cast<const uint32_t(*)[32]>(&pa[32 * c]));
         tmem_st_wait();
         tc_fence_before_sync();
         mbar_arrive(p_full(g));
@@ -690,7 +714,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       const int rows_owned = unit_rows / S;
       const uint32_t owner = softmax_thread ? static_cast<uint32_t>(grow / rows_owned) : 0u;
       const int lrow = grow % rows_owned;
-      const uint32_t recv = smem_base + AttnSmem::kK;
+      const uint32_t recv = smem_base + Shape::kK;
       if (softmax_thread && owner != crank && fin_valid) {
         const uint32_t slot = (crank < owner) ? crank : crank - 1;
         const uint32_t base = map_to_cta(recv + ((slot * 66u) * rows_owned + lrow) * 4u, owner);
@@ -702,7 +726,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attention_kernel(const __grid
       }
       cluster_sync_all();  // all partials have landed
       if (softmax_thread && owner == crank && fin_valid) {
-        const float* rbuf = reinterpret_cast<const float*>(smem_gen + AttnSmem::kK);
+        const float* rbuf = reinterpret_cast<const float*>(smem_gen + Shape::kK);
         float m_all = fin_m;
         for (int s2 = 0; s2 < S - 1; ++s2) m_all = fmaxf(m_all, rbuf[(s2 * 66 + 65) * rows_owned + lrow]);
         const float own_scale = fast_exp2(fin_m - m_all);
@@ -886,8 +910,66 @@ __global__ void __launch_bounds__(kShortThreads, 512 / kShortKeys) attention_sho
   }
 }
 
-static int g_attn_clusters[64][5] = {};
-static int g_force_attn_split = 0;  // test hook: 0 = choose
+static int g_force_attn_split = 0, g_force_attn_groups = 0, g_force_attn_keys = 0;  // test hooks: 0 = choose
+
+// Tokens per key tile, query tiles per unit and K/V split: least rounds x time of a round.  Three groups of 64-token tiles
+// keep the softmax units busiest; where a round has work for fewer query tiles than that (strips: few queries
+// against the keys of all strips), two of 128 tokens spend less on each key, as one wait and one publication of P
+// serve twice the keys.  A unit of fewer query tiles takes not much less time, it only fills more CTAs.  Without a
+// split a CTA walks several units; with one each cluster serves one unit and merges.  The times (us per key tile by
+// query tiles in it, per unit, per call) are a least-squares fit over 51 shapes (1 to 20 x 2 heads, 64 to 16384
+// queries, 1 to 8 slots, 144 to 16384 keys) x 15 combinations; the choice is 0.5 % slower than the best of the 15 on
+// average, 6 % at most.  2 x 20 heads: 512 queries of 2 strips 21.6 -> 18.7 us, 1208 of 4 138 -> 115, 128 of 8
+// 15.9 -> 11.7; 2 x 10 heads: 512 of 8 40.4 -> 33.5 (64-token tiles alone -> both).
+struct AttnPlan {
+  int keys, groups, split;
+  double us;
+};
+struct AttnCosts {
+  double tile[4];        // per key tile, by query tiles
+  double unit[5];        // per unit, by split
+};
+static constexpr AttnCosts kCosts64{{0.0, 0.685, 1.099, 1.261}, {0.0, 3.01, 4.99, 0.0, 5.56}};
+static constexpr AttnCosts kCosts128{{0.0, 1.104, 1.608, 0.0}, {0.0, 2.90, 5.30, 0.0, 5.92}};
+
+template <int kGroups, int kTileKV>
+static void plan_attention(const AttnCosts& costs, int heads_b, int q_tiles, int n_slots, int L_slot, AttnPlan& best) {
+  static int resident[64][5] = {};
+  using Shape = AttnShape<kGroups, kTileKV>;
+  if (g_force_attn_keys && g_force_attn_keys != kTileKV) return;
+  const int total_tiles = n_slots * ((L_slot + kTileKV - 1) / kTileKV);
+  int at_once[5] = {0, sm_count(), 0, 0, 0};
+  for (int w = 2; w <= 4; w *= 2) at_once[w] = resident_clusters(attention_kernel<kGroups, kTileKV>, Shape::kThreads, Shape::kTotal, w, resident);
+  for (int g = 1; g <= kGroups; ++g) {
+    if (g_force_attn_groups ? g != g_force_attn_groups : g > q_tiles) continue;
+    const int work = ((q_tiles + g - 1) / g) * heads_b;
+    for (int s2 = 1; s2 <= 4 && s2 <= total_tiles; s2 *= 2) {
+      if (g_force_attn_split && s2 != g_force_attn_split) continue;
+      const int rounds = (work + at_once[s2] - 1) / at_once[s2];
+      const double us = 1.5 + rounds * (((total_tiles + s2 - 1) / s2) * costs.tile[g < q_tiles ? g : q_tiles] + costs.unit[s2]);
+      if (best.keys == 0 || us < best.us) best = AttnPlan{kTileKV, g, s2, us};
+    }
+  }
+}
+
+template <int kGroups, int kTileKV>
+static int launch_attention(AttnParams& p, const AttnPlan& plan, int q_tiles, cudaStream_t stream) {
+  using Shape = AttnShape<kGroups, kTileKV>;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(attention_kernel<kGroups, kTileKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kTotal),
+                            "cudaFuncSetAttribute(attention)"))
+      return rc;
+    configured[dev] = true;
+  }
+  p.kv_split = plan.split, p.groups = plan.groups;
+  const int work = ((q_tiles + plan.groups - 1) / plan.groups) * p.heads * p.B;
+  const int grid = (plan.split == 1) ? (work < sm_count() ? work : sm_count()) : work * plan.split;
+  return launch_kernel("attention_kernel launch", attention_kernel<kGroups, kTileKV>, dim3(grid), dim3(Shape::kThreads), Shape::kTotal, stream,
+                       plan.split, p);
+}
 
 static int launch_short(const AttnParams& p, cudaStream_t stream) {
   static bool configured[64] = {};
@@ -914,6 +996,13 @@ extern "C" int bxl_debug_force_attn_split(int split) {
   return kOk;
 }
 
+extern "C" int bxl_debug_force_attn_tiles(int groups, int keys) {
+  if (groups < 0 || groups > 3 || (keys != 0 && keys != 64 && keys != 128) || (keys == 128 && groups > 2))
+    return fail(kErrInvalidArg, "bxl_debug_force_attn_tiles: 0..3 query tiles (2 of 128 keys), 0, 64 or 128 keys");
+  g_force_attn_groups = groups, g_force_attn_keys = keys;
+  return kOk;
+}
+
 extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long ld_q, const void* const* kv_slots,
                                 int n_slots, long long kv_img_stride, long long ld_kv, int v_col0, void* out,
                                 long long out_img_stride, long long ld_out, int B, int heads, int L_q, int L_slot,
@@ -937,14 +1026,22 @@ extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long
     uint32_t box[3] = {kHeadDim, kTileQ, 1};
     if (int rc = encode_tmap_f16(&p.q_map, q, 3, dims, str, box)) return rc;
   }
-  // attention_short_kernel is the faster one at every measured size that it serves; a forced K/V split means the other
-  const bool few_keys = n_slots == 1 && L_slot <= kShortKeys && !g_force_attn_split;
+  // attention_short_kernel is the faster one at every measured size that it serves; a forced plan means the other
+  const bool few_keys = n_slots == 1 && L_slot <= kShortKeys && !g_force_attn_split && !g_force_attn_groups && !g_force_attn_keys;
+  const int q_tiles = (L_q + kTileQ - 1) / kTileQ;
+  AttnPlan plan{0, 0, 0, 0.0};
+  if (!few_keys) {
+    plan_attention<3, 64>(kCosts64, heads * B, q_tiles, n_slots, L_slot, plan);
+    plan_attention<2, 128>(kCosts128, heads * B, q_tiles, n_slots, L_slot, plan);
+    if (plan.keys == 0 && !g_force_attn_groups && !g_force_attn_keys) plan = AttnPlan{64, q_tiles < 3 ? q_tiles : 3, 1, 0.0};   // more splits forced than key tiles
+    if (plan.keys == 0) return fail(kErrInvalidArg, "bxl_attn_fwd_f16: the forced tiles and split do not fit %d slots of %d keys", n_slots, L_slot);
+  }
   for (int s = 0; s < (few_keys ? 1 : kMaxSlots); ++s) {
     const void* base = kv_slots[s < n_slots ? s : 0];
     if (!base) return fail(kErrInvalidArg, "bxl_attn_fwd_f16: slot %d null", s);
     uint64_t dims[3] = {(uint64_t)(v_col0 + heads * kHeadDim), (uint64_t)L_slot, (uint64_t)B};
     uint64_t str[2] = {(uint64_t)ld_kv * 2, (uint64_t)kv_img_stride * 2};
-    uint32_t box[3] = {kHeadDim, (uint32_t)(few_keys ? (L_slot + 15) / 16 * 16 : kTileKV), 1};
+    uint32_t box[3] = {kHeadDim, (uint32_t)(few_keys ? (L_slot + 15) / 16 * 16 : plan.keys), 1};
     if (int rc = encode_tmap_f16(&p.kv_map[s], base, 3, dims, str, box)) return rc;
   }
   p.n_slots = n_slots, p.L_q = L_q, p.L_slot = L_slot, p.heads = heads, p.B = B, p.v_col0 = v_col0;
@@ -953,41 +1050,6 @@ extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long
   p.scale_log2e = scale * 1.4426950408889634f;
   p.dev_status = st;
   if (few_keys) return launch_short(p, (cudaStream_t)stream);
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem::kTotal),
-                            "cudaFuncSetAttribute(attention)"))
-      return rc;
-    configured[dev] = true;
-  }
-  // Query tiles per unit and K/V split: fewest rounds x time of a round, in K/V tiles of a full unit (1.2 us).  A
-  // unit of fewer query tiles takes not much less time (its softmax warps then share the special-function units
-  // with fewer others), it only fills more CTAs.  Without a split a CTA walks several units and pays ~1.5 tiles of
-  // bubble per unit; with a split each cluster serves one unit and pays ~6.5 tiles of set-up and merge.  Over 20
-  // shapes (64 to 16384 queries, 77 to 16384 keys) the choice is the fastest of the nine combinations or within 4 %.
-  const int q_tiles = (L_q + kTileQ - 1) / kTileQ;
-  const int total_tiles = n_slots * ((L_slot + kTileKV - 1) / kTileKV);
-  static const double kTileCost[kGroups + 1] = {0.0, 0.58, 0.85, 1.0};
-  int split = 1, groups = kGroups;
-  double best = 1e30;
-  int at_once[5] = {0, sm_count(), 0, 0, 0};
-  for (int w = 2; w <= 4; w *= 2) at_once[w] = resident_clusters(attention_kernel, kAttnThreads, AttnSmem::kTotal, w, g_attn_clusters);
-  for (int g = kGroups; g >= 1; --g) {
-    const int work = ((q_tiles + g - 1) / g) * heads * B;
-    for (int s2 = 1; s2 <= 4; s2 *= 2) {
-      if (s2 > total_tiles || (g_force_attn_split && s2 != g_force_attn_split)) continue;
-      const int clusters = at_once[s2];
-      const int rounds = (work + clusters - 1) / clusters;
-      const double tc = kTileCost[g < q_tiles ? g : (q_tiles < kGroups ? q_tiles : kGroups)];
-      const double cost = (s2 == 1) ? rounds * (total_tiles * tc + 1.5) : rounds * (((total_tiles + s2 - 1) / s2) * tc + 6.5);
-      if (cost < best - 1e-9) best = cost, split = s2, groups = g;
-    }
-  }
-  p.kv_split = split, p.groups = groups;
-  const int work = ((q_tiles + groups - 1) / groups) * heads * B;
-  const int grid = (split == 1) ? (work < sm_count() ? work : sm_count()) : work * split;
-  return launch_kernel("attention_kernel launch", attention_kernel, dim3(grid), dim3(kAttnThreads), AttnSmem::kTotal,
-                       (cudaStream_t)stream, split, p);
+  return plan.keys == 128 ? launch_attention<2, 128>(p, plan, q_tiles, (cudaStream_t)stream)
+                          : launch_attention<3, 64>(p, plan, q_tiles, (cudaStream_t)stream);
 }

@@ -68,6 +68,11 @@ int bxl_debug_force_tile_order(int order);
  * 0 restores the built-in choice).  No counterpart in the reference. */
 int bxl_debug_force_attn_split(int split);
 
+/* Test hook: force the query tiles per work unit (1, 2 or 3; at most 2 with 128-token key tiles) and the tokens per
+ * key tile (64 or 128) of the attention kernel; 0 restores the built-in choice.  With either forced, a call that the
+ * forced plan (K/V split included) does not fit returns an error.  No counterpart in the reference. */
+int bxl_debug_force_attn_tiles(int groups, int keys);
+
 /* ---- matmul ------------------------------------------------------------- */
 
 /* C[M,N] = A[M,K] * B (+ bias[N]) (+ residual[M,N]); fp16 operands, fp32

@@ -1,5 +1,6 @@
 """Flash-style attention kernel through the C ABI against the CPU oracle and the
 fixtures produced by the reference module."""
+import contextlib
 import os
 
 import numpy as np
@@ -20,6 +21,25 @@ def _ops():
     return _lib, ops
 
 
+@contextlib.contextmanager
+def _plan(keys, groups, split):
+    """Forces tokens per key tile, query tiles per work unit and K/V split (0 = the kernel's choice)."""
+    _lib, _ = _ops()
+    l = _lib.lib()
+    _lib.check(l.bxl_debug_force_attn_tiles(groups, keys), l, kernels=0)
+    _lib.check(l.bxl_debug_force_attn_split(split), l, kernels=0)
+    try:
+        yield
+        _lib.device_status()
+    finally:
+        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
+        _lib.check(l.bxl_debug_force_attn_tiles(0, 0), l, kernels=0)
+
+
+# every tile width, count of groups at work and split, some forced, some chosen
+PLANS = [(0, 0, 0), (64, 3, 1), (64, 3, 2), (64, 3, 4), (64, 2, 1), (64, 2, 4), (64, 1, 2), (128, 2, 1), (128, 2, 2), (128, 2, 4), (128, 1, 1), (128, 1, 4)]
+
+
 @pytest.mark.parametrize(
     "B,heads,Lq,Lslot,nslots",
     [
@@ -28,14 +48,14 @@ def _ops():
         (1, 2, 256, 128, 3),
         (2, 10, 77, 77, 1),       # ragged query and key tiles
         (2, 10, 512, 77, 1),      # cross-attention: 77 text tokens
-        (2, 20, 1024, 128, 2),    # 160 work units on 148 SMs: the under-filled second round runs as half units
-        (2, 20, 1024, 77, 1),     # the same count for cross-attention
+        (2, 20, 1024, 128, 2),    # 320 query tiles
+        (2, 20, 1024, 77, 1),     # the same count for cross-attention: a CTA each
         (1, 3, 200, 72, 4),       # ragged slots
         (2, 10, 512, 512, 8),     # benchmark shape at world size 8: L = 4096
         (2, 20, 256, 256, 4),     # 1280-level blocks, 4 strips
-        (2, 10, 4096, 77, 1),     # 320 units of 256 queries: every CTA walks two or three units
-        (2, 20, 1024, 256, 1),    # 160 units on 148 SMs: some CTAs walk two units of two tiles
-        (4, 20, 384, 100, 2),     # 160 units, every second one with a single query tile, ragged slots
+        (2, 10, 4096, 77, 1),     # 640 CTAs where 592 are resident
+        (2, 20, 1024, 256, 1),    # whole key tiles only, of either width
+        (4, 20, 384, 100, 2),     # three query tiles a head, ragged slots
     ],
 )
 def test_attention_core_vs_oracle(B, heads, Lq, Lslot, nslots):
@@ -120,28 +140,33 @@ def test_benchmark_shape_self_attention():
             assert_close(y, ref, what=f"self-attention strip {i} of n={n}")
 
 
+@pytest.mark.parametrize("keys,groups", [(0, 0), (64, 1), (64, 2), (64, 3), (128, 1), (128, 2)])
 @pytest.mark.parametrize("split", [1, 2, 4])
 @pytest.mark.parametrize("B,heads,Lq,Lslot,nslots", [(1, 2, 256, 128, 4), (2, 3, 200, 72, 5), (1, 20, 256, 256, 4), (2, 10, 512, 77, 1), (1, 4, 640, 512, 2)])
-def test_attention_kv_split_over_a_cluster(B, heads, Lq, Lslot, nslots, split):
+def test_attention_kv_split_over_a_cluster(B, heads, Lq, Lslot, nslots, split, keys, groups):
     """The K/V range split over 1, 2 or 4 CTAs per query block and merged through distributed
-    shared memory gives the same result (ragged tiles, several slots, odd query-tile counts)."""
+    shared memory gives the same result (ragged tiles, several slots, odd query-tile counts, one to three
+    query tiles whose rows the CTAs of the cluster share out)."""
     dev = cuda_or_skip()
     _lib, ops = _ops()
-    if split > nslots * ((Lslot + 127) // 128):
+    if split > nslots * -(-Lslot // (keys or 64)):
         pytest.skip("more splits than key/value tiles")
     C = heads * 64
     gen = torch.Generator().manual_seed(B + heads + Lq + Lslot + nslots)
     q = h16(torch.randn(B, Lq, C, generator=gen))
     slots = [h16(torch.randn(B, Lslot, 2 * C, generator=gen) * (1.0 + 2.0 * i)) for i in range(nslots)]  # very different maxima per slot
     ref = po._sdpa_heads(q, torch.cat(slots, dim=1), heads)
-    l = _lib.lib()
-    _lib.check(l.bxl_debug_force_attn_split(split), l, kernels=0)
-    try:
+    with _plan(keys, groups, split):
         y = ops.attention(q.half().to(dev), [s.half().to(dev) for s in slots], heads)
-        _lib.device_status()
-    finally:
-        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
-    assert_close(y, ref, tol=3e-3, what=f"attention split={split}")
+    assert_close(y, ref, tol=3e-3, what=f"attention split={split} keys={keys} groups={groups}")
+
+
+def test_a_forced_plan_that_does_not_fit_is_refused():
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    q, kv = torch.zeros(1, 300, 64, dtype=torch.float16, device=dev), torch.zeros(1, 100, 128, dtype=torch.float16, device=dev)
+    with pytest.raises(_lib.BxlError, match="forced"), _plan(128, 2, 2):
+        ops.attention(q, [kv], 1)
 
 
 def test_self_attention_at_16384_tokens():
@@ -162,47 +187,42 @@ def test_self_attention_at_16384_tokens():
     assert_close(y, ref, what="self-attention L=16384")
 
 
-@pytest.mark.parametrize("split", [0, 1, 2])
-@pytest.mark.parametrize("Lq", [1, 128, 129, 257, 384, 385, 513, 770])
-@pytest.mark.parametrize("Lslot,nslots", [(1, 3), (63, 1), (64, 2), (65, 2), (200, 8)])
-def test_attention_tile_edges(Lq, Lslot, nslots, split):
-    """One to three query tiles per unit with the last one ragged, key tiles that end on, before and after a
-    64-token boundary, and more than one ring's worth of them."""
+@pytest.mark.parametrize("keys,groups,split", PLANS)
+@pytest.mark.parametrize("Lq", [1, 128, 129, 257, 385, 770])
+@pytest.mark.parametrize("Lslot,nslots", [(1, 3), (63, 2), (64, 4), (65, 2), (127, 2), (129, 4), (200, 8)])
+def test_attention_tile_edges(Lq, Lslot, nslots, keys, groups, split):
+    """One to three query tiles per unit with the last one ragged, key tiles that end on, before and after a 64- and a
+    128-token boundary, more than one ring's worth of them, and clusters that merge the rows of every such unit."""
     dev = cuda_or_skip()
     _lib, ops = _ops()
+    if split > nslots * -(-Lslot // (keys or 64)):
+        pytest.skip("more splits than key/value tiles")
     B, heads = 2, 3
     C = heads * 64
     gen = torch.Generator().manual_seed(Lq + 1000 * Lslot + nslots)
     q = h16(torch.randn(B, Lq, C, generator=gen))
     slots = [h16(torch.randn(B, Lslot, 2 * C, generator=gen)) for _ in range(nslots)]
     ref = po._sdpa_heads(q, torch.cat(slots, dim=1), heads)
-    l = _lib.lib()
-    _lib.check(l.bxl_debug_force_attn_split(split), l, kernels=0)
-    try:
+    with _plan(keys, groups, split):
         y = ops.attention(q.half().to(dev), [s.half().to(dev) for s in slots], heads)
-        _lib.device_status()
-    finally:
-        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
-    assert_close(y, ref, what=f"attention Lq{Lq} Ls{Lslot} n{nslots} split{split}")
+    assert_close(y, ref, what=f"attention Lq{Lq} Ls{Lslot} n{nslots} keys{keys} groups{groups} split{split}")
 
 
-def test_attention_walks_many_units():
-    """More units than CTAs, the last unit of every head with one tile: the groups' barriers and the rings of
+@pytest.mark.parametrize("keys,groups,Lq", [(64, 3, 4 * 384 + 60), (128, 2, 6 * 256 + 60), (64, 2, 6 * 256 + 60)])
+def test_attention_walks_many_units(keys, groups, Lq):
+    """Two or more units for every CTA, the last unit of every head with one tile: the groups' barriers and the rings of
     keys and queries go round many times, with idle groups in between."""
     dev = cuda_or_skip()
     _lib, ops = _ops()
-    B, heads, Lq, Lslot = 2, 20, 4 * 384 + 60, 150
+    B, heads, Lslot = 2, 40, 150
     C = heads * 64
+    units = B * heads * -(-Lq // (128 * groups))
+    assert units >= 2 * _lib.lib().bxl_sm_count()
     gen = torch.Generator().manual_seed(9)
     q, kv = h16(torch.randn(B, Lq, C, generator=gen)), h16(torch.randn(B, Lslot, 2 * C, generator=gen))
     ref = po._sdpa_heads(q, kv, heads)
-    l = _lib.lib()
-    _lib.check(l.bxl_debug_force_attn_split(1), l, kernels=0)
-    try:
+    with _plan(keys, groups, 1):
         y = ops.attention(q.half().to(dev), [kv.half().to(dev)], heads)
-        _lib.device_status()
-    finally:
-        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
     assert_close(y, ref, what="attention, many units")
 
 
@@ -249,25 +269,22 @@ def test_attention_error_with_peaked_scores(L):
     assert got <= 1.02 * err(model), f"{got:.4e} > 1.02 * {err(model):.4e}"
 
 
-@pytest.mark.parametrize("split", [0, 1, 2, 4])
-@pytest.mark.parametrize("masked", [1, 63, 64, 65, 128, 129, 200, 319, 320])
-def test_attention_after_keys_of_minus_infinity(masked, split):
+@pytest.mark.parametrize("keys,groups,split", PLANS)
+@pytest.mark.parametrize("masked,total", [(1, 320), (63, 320), (64, 320), (65, 320), (128, 320), (129, 320), (200, 320), (319, 320), (320, 320), (70, 100), (100, 100)])
+def test_attention_after_keys_of_minus_infinity(masked, total, keys, groups, split):
     """Keys whose scores are -inf (a mask feature, left padding) weigh nothing, however many come first; a row that has
     no other key is NaN."""
     dev = cuda_or_skip()
     _lib, ops = _ops()
     gen = torch.Generator().manual_seed(masked)
-    q, kv = h16(torch.randn(1, 200, 128, generator=gen)), h16(torch.randn(1, 320, 256, generator=gen))
+    q, kv = h16(torch.randn(1, 200, 128, generator=gen)), h16(torch.randn(1, total, 256, generator=gen))
     q[..., 5] = q[..., 70] = 1.0
     kv[0, :masked, 5] = kv[0, :masked, 70] = float("-inf")
-    l = _lib.lib()
-    _lib.check(l.bxl_debug_force_attn_split(split), l, kernels=0)
-    try:
+    if split > -(-total // (keys or 64)):
+        pytest.skip("more splits than key/value tiles")
+    with _plan(keys, groups, split):
         y = ops.attention(q.half().to(dev), [kv.half().to(dev)], 2)
-        _lib.device_status()
-    finally:
-        _lib.check(l.bxl_debug_force_attn_split(0), l, kernels=0)
-    if masked == 320:
+    if masked == total:
         assert torch.isnan(y).all()
     else:
         assert_close(y, po._sdpa_heads(q, kv[:, masked:], 2), what=f"{masked} keys of -inf first, split {split}")
