@@ -245,10 +245,15 @@ struct GnFusedParams {
 // kDepth: pixels a thread loads before it uses the first.  8 where one CTA has an SM and a thread has 16 pixels or more,
 // so that what is in flight covers the latency: 2 x 320 x 256 x 256 180 -> 90 us, 2 x 960 x 128 x 128 128 -> 61, 2 x 320 x
 // 128 x 128 37.2 -> 33.6; 4 elsewhere, where deeper loads made the short passes slower (2 x 640 x 64 x 64 17.9 -> 20.8).
-template <int kDepth>
+// kSlab: whether the slab stays in shared memory is known at compile time for short passes, where the branches count
+// (2 x 1920 x 48 x 46 23.9 -> 20.6 us, 2 x 640 x 64 x 64 18.6 -> 17.5, 2 x 1280 x 8 x 32 9.1 -> 8.7); from 9 pixels a thread on
+// the code that asks p.keep is the faster one (2 x 640 x 128 x 128 52.4 -> 48.9, 2 x 1920 x 64 x 64 49.3 -> 46.3).
+enum GnSlab { kReread, kKept, kAsked };
+template <int kDepth, GnSlab kSlab>
 __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParams p) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) unsigned char gnf_smem[];
+  const bool keep = kSlab == kAsked ? p.keep != 0 : kSlab == kKept;
   const int cb = p.cb, bv = cb / 8, cpg = p.C / p.G, gb = cb / cpg;
   const int rows = blockDim.x / bv;                       // pixels per sweep
   const uint32_t crank = p.cs > 1 ? cluster_ctarank() : 0u;
@@ -290,13 +295,13 @@ __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParam
       for (int j = 0; j < kDepth; ++j) u[j] = __ldg(reinterpret_cast<const uint4*>(xb + (long long)(pix + j * rows) * p.C));
 #pragma unroll
       for (int j = 0; j < kDepth; ++j) {
-        if (p.keep) s_slab[(size_t)(pix + j * rows - p0) * bv + v] = u[j];
+        if (keep) s_slab[(size_t)(pix + j * rows - p0) * bv + v] = u[j];
         accumulate8(u[j], s1, s2);
       }
     }
     for (; pix < p1; pix += rows) {
       const uint4 u = __ldg(reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
-      if (p.keep) s_slab[(size_t)(pix - p0) * bv + v] = u;
+      if (keep) s_slab[(size_t)(pix - p0) * bv + v] = u;
       accumulate8(u, s1, s2);
     }
     float* d1 = s_part + ((size_t)r * 2) * cb + v * 8;
@@ -404,14 +409,15 @@ __global__ void __launch_bounds__(512) groupnorm_fused_kernel(const GnFusedParam
         *reinterpret_cast<uint4*>(p.halo_out + (((long long)p.B + img) * p.W + (pix - last_row0)) * p.C + (long long)cblk * cb + v * 8) = o;
     }
   };
-  if (kDepth <= 4) {
+  if (kDepth <= 4 && kSlab != kReread) {
     for (int pix = p0 + r; pix < p1; pix += rows)
-      normalise(pix, p.keep ? s_slab[(size_t)(pix - p0) * bv + v] : *reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
-  } else if (p.keep) {
+      normalise(pix, keep ? s_slab[(size_t)(pix - p0) * bv + v] : *reinterpret_cast<const uint4*>(xb + (long long)pix * p.C));
+  } else if (keep) {
 #pragma unroll 2
     for (int pix = p0 + r; pix < p1; pix += rows) normalise(pix, s_slab[(size_t)(pix - p0) * bv + v]);
   } else {
-    // from the end of the slab, which the first pass has read last: more of it is still in L2
+    // from the end of the slab, which the first pass has read last: more of it is still in L2 (2 x 1920 x 254 x 143,
+    // several CTAs on an SM: 298 -> 204 us)
     int n = (p1 - p0 - r + rows - 1) / rows;   // this thread's pixels (none if not positive)
     for (; n >= kDepth; n -= kDepth) {
       const int last = p0 + r + (n - 1) * rows;
@@ -557,7 +563,7 @@ extern "C" int bxl_groupnorm_fused_f16(const void* x, void* y, long long img_str
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    for (auto kernel : {groupnorm_fused_kernel<4>, groupnorm_fused_kernel<8>})
+    for (auto kernel : {groupnorm_fused_kernel<4, kReread>, groupnorm_fused_kernel<4, kKept>, groupnorm_fused_kernel<4, kAsked>, groupnorm_fused_kernel<8, kAsked>})
       if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024),
                               "cudaFuncSetAttribute(groupnorm_fused)"))
         return rc;
@@ -568,7 +574,10 @@ extern "C" int bxl_groupnorm_fused_f16(const void* x, void* y, long long img_str
   p.fresh_out = fresh_out, p.n_peers = mode == 2 ? n_peers : 0, p.own = own, p.mode = mode, p.eps = eps;
   p.gamma = static_cast<const __half*>(gamma), p.beta = static_cast<const __half*>(beta), p.silu = silu;
   p.halo_out = static_cast<__half*>(halo_out), p.W = W;
-  auto kernel = (long long)cs * nblk * B <= sm_count() && per * bv >= 16 * threads ? groupnorm_fused_kernel<8> : groupnorm_fused_kernel<4>;
+  auto kernel = (long long)cs * nblk * B <= sm_count() && per * bv >= 16 * threads ? groupnorm_fused_kernel<8, kAsked>
+                : !keep                                                            ? groupnorm_fused_kernel<4, kReread>
+                : per * bv >= 9 * threads                                          ? groupnorm_fused_kernel<4, kAsked>
+                                                                                   : groupnorm_fused_kernel<4, kKept>;
   return launch_kernel("groupnorm_fused_kernel launch", kernel, dim3(cs * nblk, B), dim3(threads), smem,
                        (cudaStream_t)stream, cs, p);
 }

@@ -173,6 +173,31 @@ def test_groupnorm_fused_config_shapes(C, H, W, n):
     _lib.device_status()
 
 
+@pytest.mark.parametrize("C,H,W", [
+    (1920, 77, 75),    # slab re-read, several CTAs on an SM: from its end, four pixels at a time and a remainder
+    (960, 131, 127),   # slab re-read, one CTA on an SM, eight at a time
+    (1920, 63, 61),    # slab kept, nine pixels a thread or more
+    (320, 127, 125),   # slab kept, eight loads in flight
+    (1920, 48, 46),    # slab kept, fewer than nine
+    (960, 13, 12),     # two or three pixels a thread, uneven ranges
+])
+def test_groupnorm_fused_slab_forms(C, H, W):
+    """Every form of the second pass, at sizes that leave remainders in it, against the oracle; twice the same bits."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    gen = torch.Generator().manual_seed(C + H)
+    x = h16(torch.randn(2, C, H, W, generator=gen) * 2 + 0.5)
+    gamma, beta = torch.randn(C, generator=gen), torch.randn(C, generator=gen)
+    ref = po.groupnorm_pp(x, 32, 1e-5, h16(gamma), h16(beta), None, 0, "local")
+    y, m, halo = _run_fused(ops, dev, x, 32, 1e-5, gamma, beta, None, 0, "local", halo=True)
+    assert_close(y, ref, what=f"fused gn {C}x{H}x{W}")
+    assert_close(m.cpu().reshape(-1), po.groupnorm_moments(x, 32).reshape(-1), tol=1e-3, what="fused gn moments")
+    assert torch.equal(halo[0, :, 0], nhwc(y)[:, 0]) and torch.equal(halo[1, :, 0], nhwc(y)[:, -1])
+    again, _, _ = _run_fused(ops, dev, x, 32, 1e-5, gamma, beta, None, 0, "local")
+    assert torch.equal(y, again)
+    _lib.device_status()
+
+
 def test_groupnorm_fused_negative_variance_fallback():
     dev = cuda_or_skip()
     _lib, ops = _ops()
