@@ -207,15 +207,20 @@ def gemm_fused(a, w, *, bias=None, bias_f32=None, residual=None, out=None, out2=
 
 
 def gemm_ragged(a, b, bias=None, residual=None):
-    """``a[M,K] @ b[K,N] (+ bias) (+ residual)`` for matrices whose rows are not 16-byte aligned.  ``b`` is
-    contiguous; the rows of ``a`` and ``residual`` are unit-stride, any distance apart."""
+    """``a[M,K] @ b[K,N] (+ bias) (+ residual)`` for matrices whose rows are not 16-byte aligned.  ``b`` and
+    ``bias`` (``[N]``) are contiguous; the rows of ``a`` and ``residual`` are unit-stride, any distance apart."""
     _f16_cuda(a, "a"), _f16_cuda(b, "b")
+    _req(a.dim() == 2 and b.dim() == 2 and a.device == b.device, "gemm_ragged: 2-D operands on one device")
     M, K = a.shape
     N = b.shape[1]
     _req(b.shape[0] == K, "gemm_ragged: inner dimensions differ")
+    _req((K == 1 or a.stride(1) == 1) and b.is_contiguous(), "gemm_ragged: row-major a, contiguous b")
     if residual is not None:
         _f16_cuda(residual, "residual")
-        _req(residual.shape == (M, N), "gemm_ragged: bad residual")
+        _req(residual.shape == (M, N) and (N == 1 or residual.stride(1) == 1) and residual.device == a.device, "gemm_ragged: bad residual")
+    if bias is not None:
+        _f16_cuda(bias, "bias")
+        _req(bias.shape == (N,) and bias.is_contiguous() and bias.device == a.device, "gemm_ragged: bad bias")
     out = torch.empty((M, N), device=a.device, dtype=torch.float16)
     l = _lib.lib()
     ws = torch.empty(max(l.bxl_gemm_ragged_workspace_bytes(M, N, K), 16), device=a.device, dtype=torch.uint8)
