@@ -56,15 +56,18 @@ def cascaded_lowp_matmul(
             return out
         return res.reshape(*batch_dims, N)
     if K % 8 or N % 8:
-        # the kernel adds a plain fp16 row of N values; any other bias is added to the product
-        fused = bias if bias is not None and bias.is_cuda and bias.dtype == torch.float16 and bias.shape == (N,) and bias.stride(0) == 1 else None
-        r2 = None if residual is None else residual.reshape(-1, N)
+        # the kernel adds a plain fp16 row of N values and an fp16 matrix; any other bias or residual is added to the product
+        fits = lambda t: t is not None and t.dtype == torch.float16 and t.device == a.device
+        fused = bias if fits(bias) and bias.shape == (N,) and bias.stride(0) == 1 else None
+        r2 = residual.reshape(-1, N) if fits(residual) and residual.numel() == a2.shape[0] * N else None
         if r2 is not None and r2.stride(1) != 1:
             r2 = r2.contiguous()
         res = ops.gemm_ragged(a2, b, bias=fused, residual=r2)
         if bias is not None and fused is None:
             res = res + bias
         res = res.reshape(*batch_dims, N)
+        if residual is not None and r2 is None:
+            res = (res + residual.to(res.device)).to(res.dtype)
         if out is not None:
             out.copy_(res)
             return out

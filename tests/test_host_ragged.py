@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from basedxl_b200 import _lib, ops
+from basedxl_b200.cascaded_lowp_matmul import cascaded_lowp_matmul
 
 
 class _Recorder:
@@ -76,3 +77,32 @@ def test_operands_that_the_kernel_reads_are_passed_on(recorder, kw, lda, ldr):
     assert ops.gemm_ragged(**args).shape == (5, 9)
     (call,) = recorder.calls
     assert (call[1], call[3], call[6]) == (lda, 9, ldr) and call[9:12] == (5, 9, args["a"].shape[1])
+
+
+@pytest.fixture
+def product(monkeypatch):
+    """The kernel replaced by PyTorch, with the operands it takes."""
+
+    def gemm_ragged(a, b, bias=None, residual=None):
+        for t in (bias, residual):
+            ops._req(t is None or t.dtype == torch.float16, "gemm_ragged: expected fp16")
+        y = a.float() @ b.float()
+        y = y if bias is None else y + bias.detach().float()
+        return (y if residual is None else y + residual.float()).half()
+
+    monkeypatch.setattr(ops, "gemm_ragged", gemm_ragged)
+
+
+@pytest.mark.parametrize("bias_type", [None, torch.float16, torch.float32])
+@pytest.mark.parametrize("residual", ["fp16", "fp32", "one row", "one value", "transposed"])
+def test_any_residual_is_added(product, residual, bias_type):
+    """Whatever its type and broadcast, and whatever the bias is."""
+    g = torch.Generator().manual_seed(1)
+    a, b = torch.randn(2, 5, 7, generator=g).half(), torch.randn(7, 9, generator=g).half()
+    full = torch.randn(2, 5, 9, generator=g).half()
+    r = {"fp16": full, "fp32": full.float(), "one row": full[0, 0], "one value": full[0, 0, :1], "transposed": full.transpose(1, 2).contiguous().transpose(1, 2)}[residual]
+    bias = None if bias_type is None else torch.randn(9, generator=g).to(bias_type)
+    y = cascaded_lowp_matmul(a, b, bias=bias, residual=r)
+    ref = a.float() @ b.float() + r.float() + (0 if bias is None else bias.float())
+    assert y.shape == (2, 5, 9) and y.dtype == (torch.float32 if bias_type == torch.float32 else torch.float16)
+    assert float((y.float() - ref).abs().max()) <= 3 * 2.0**-11 * float(ref.abs().max() + 4)
