@@ -58,7 +58,7 @@ def cascaded_lowp_matmul(
     if K % 8 or N % 8:
         # the kernel adds a plain fp16 row of N values and an fp16 matrix; any other bias or residual is added to the product
         fits = lambda t: t is not None and t.dtype == torch.float16 and t.device == a.device
-        fused = bias if fits(bias) and bias.shape == (N,) and bias.stride(0) == 1 else None
+        fused = bias if fits(bias) and bias.shape == (N,) and bias.stride(0) == 1 and not (bias.requires_grad and torch.is_grad_enabled()) else None
         r2 = residual.reshape(-1, N) if fits(residual) and residual.numel() == a2.shape[0] * N else None
         if r2 is not None and r2.stride(1) != 1:
             r2 = r2.contiguous()

@@ -106,3 +106,12 @@ def test_any_residual_is_added(product, residual, bias_type):
     ref = a.float() @ b.float() + r.float() + (0 if bias is None else bias.float())
     assert y.shape == (2, 5, 9) and y.dtype == (torch.float32 if bias_type == torch.float32 else torch.float16)
     assert float((y.float() - ref).abs().max()) <= 3 * 2.0**-11 * float(ref.abs().max() + 4)
+
+
+def test_gradient_of_a_bias(product):
+    """A bias that asks for a gradient gets it from unaligned extents, as the sum outside the kernel gives it."""
+    bias = torch.zeros(9, dtype=torch.float16, requires_grad=True)
+    cascaded_lowp_matmul(_h(5, 7), _h(7, 9), bias=bias).float().sum().backward()
+    assert torch.equal(bias.grad, torch.full((9,), 5.0, dtype=torch.float16))
+    with torch.no_grad():
+        assert not cascaded_lowp_matmul(_h(5, 7), _h(7, 9), bias=bias).requires_grad
