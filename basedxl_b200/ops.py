@@ -222,12 +222,14 @@ def gemm_ragged(a, b, bias=None, residual=None):
         _f16_cuda(bias, "bias")
         _req(bias.shape == (N,) and bias.is_contiguous() and bias.device == a.device, "gemm_ragged: bad bias")
     out = torch.empty((M, N), device=a.device, dtype=torch.float16)
+    # operands whose rows are not 16-byte aligned (or overlap) are copied by a launch of their own
+    copied = any(t.data_ptr() % 16 or ld % 8 or ld < t.shape[1] for t, ld in ((a, a.stride(0)), (b, N)))
     l = _lib.lib()
     ws = torch.empty(max(l.bxl_gemm_ragged_workspace_bytes(M, N, K), 16), device=a.device, dtype=torch.uint8)
     _lib.check(
         l.bxl_gemm_ragged_f16(_p(a), a.stride(0), _p(b), N, _p(bias), _p(residual), 0 if residual is None else residual.stride(0),
                               _p(out), N, M, N, K, _p(ws), ws.numel(), _stream()),
-        l, kernels=2,
+        l, kernels=2 if copied else 1,
     )
     return out
 

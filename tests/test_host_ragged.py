@@ -79,6 +79,23 @@ def test_operands_that_the_kernel_reads_are_passed_on(recorder, kw, lda, ldr):
     assert (call[1], call[3], call[6]) == (lda, 9, ldr) and call[9:12] == (5, 9, args["a"].shape[1])
 
 
+@pytest.mark.parametrize(
+    "a,b,launches",
+    [
+        (_h(5, 8), _h(8, 16), 1),
+        (_h(5, 16)[:, :7], _h(7, 16), 1),            # padded rows of seven
+        (_h(5, 7), _h(7, 16), 2),
+        (_h(5, 8), _h(8, 9), 2),
+        (_h(41)[1:].view(5, 8), _h(8, 16), 2),       # odd address
+        (_h(1, 8).expand(5, 8), _h(8, 16), 2),       # rows on top of one another
+    ],
+)
+def test_only_launches_that_run_are_counted(recorder, a, b, launches):
+    before = _lib.launches
+    ops.gemm_ragged(a, b)
+    assert _lib.launches - before == launches
+
+
 @pytest.fixture
 def product(monkeypatch):
     """The kernel replaced by PyTorch, with the operands it takes."""
