@@ -934,7 +934,7 @@ static constexpr AttnCosts kCosts128{{0.0, 1.104, 1.608, 0.0}, {0.0, 2.90, 5.30,
 
 template <int kGroups, int kTileKV>
 static void plan_attention(const AttnCosts& costs, int heads_b, int q_tiles, int n_slots, int L_slot, AttnPlan& best) {
-  static int resident[64][5] = {};
+  static std::atomic<int> resident[64][5] = {};
   using Shape = AttnShape<kGroups, kTileKV>;
   if (g_force_attn_keys && g_force_attn_keys != kTileKV) return;
   const int total_tiles = n_slots * ((L_slot + kTileKV - 1) / kTileKV);

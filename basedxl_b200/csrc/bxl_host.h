@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace bxl {
 
 // status codes returned over the C ABI (0 = ok, negative = error)
@@ -68,12 +70,15 @@ int launch_kernel(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 bl
 
 // Clusters of `width` CTAs that can be resident at one time, for a kernel of which an SM holds one CTA.  Fewer than
 // SMs / width: a cluster stays inside one GPC, whose SM count need not be a multiple of the width.  Asked of the
-// runtime once per device and width (`cache`: one int per width up to 4, per device).
+// runtime once per device and width (`cache`: one count per width up to 4, per device; threads that ask at the same
+// time find the same answer).  Not asked while the caller has an error pending: a failing query would take its place.
 template <typename Kernel>
-int resident_clusters(Kernel kernel, int threads, size_t smem, int width, int (*cache)[5]) {
+int resident_clusters(Kernel kernel, int threads, size_t smem, int width, std::atomic<int> (*cache)[5]) {
   int dev = 0;
+  if (cudaPeekAtLastError() != cudaSuccess) return sm_count() / width;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || width < 2 || width > 4) return sm_count() / width;
-  if (!cache[dev][width]) {
+  int known = cache[dev][width].load(std::memory_order_relaxed);
+  if (!known) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(sm_count() / width * width), cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr;
@@ -83,12 +88,13 @@ int resident_clusters(Kernel kernel, int threads, size_t smem, int width, int (*
     int n = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
+      cudaGetLastError();   // the query's own
       n = sm_count() / width;
     }
-    cache[dev][width] = n < sm_count() / width ? n : sm_count() / width;
+    known = n < sm_count() / width ? n : sm_count() / width;
+    cache[dev][width].store(known, std::memory_order_relaxed);
   }
-  return cache[dev][width];
+  return known;
 }
 
 }  // namespace bxl

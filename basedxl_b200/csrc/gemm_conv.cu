@@ -808,7 +808,7 @@ static int stages_for(int bn, int split, int pair = 0, int extra_smem = 0, int p
   return st;
 }
 
-static int g_clusters[64][5] = {};
+static std::atomic<int> g_clusters[64][5] = {};
 
 // Pick the tile width, the K split and whether to pair CTAs, minimising a time model fitted to a sweep of
 // every (tile width, split, pairing) over 110 GEMM and convolution shapes (2 to 32768 rows; both layouts of B;
