@@ -898,7 +898,11 @@ static int aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 1
 
 // test hook: force the tile width / K split (0 = choose)
 constexpr int kDefaultPair = -1;  // -1 = let the cost model decide
-constexpr double kConvAMinUs = 0.224;  // per-k-block floor of the convolution's image copies
+// Per-k-block floor of the convolution's image copies: one copy of th rows, or (stride 2) th copies of one row.  With
+// the first value for both, strided convolutions of few tiles were not split over K: 2 x 64 x 64 x 152 x 8
+// 14.1 -> 10.6 us, 1 x 128 x 128 x 16 x 90 11.7 -> 9.5, 1 x 128 x 512 x 32 x 68 11.8 -> 10.7; eleven other strided shapes
+// keep their configuration.
+static double conv_a_min_us(int stride, int th) { return stride == 1 ? 0.224 : 0.36 + 0.03 * th; }
 static int g_force_bn = 0, g_force_split = 0, g_force_pair = -1;
 static int g_force_order = -1;  // -1 = choose, 0 = consecutive tiles walk M, 1 = they walk N
 // Linear layers: an activation matrix that does not stay in L2 beside the output is walked once
@@ -1377,7 +1381,7 @@ extern "C" int bxl_conv3x3_halo_f16(const void* x, long long x_img_stride, const
   const int K = 9 * C_in;
   const int tiles_x = (W_out + tw - 1) / tw, tiles_y = (H_out + th - 1) / th;
   const TileConfig tc = choose_tiles(B * tiles_x * tiles_y, C_out, K / kBK, false, g_force_bn, g_force_split,
-                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, kConvAMinUs);
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, conv_a_min_us(stride, th));
   const int BN = tc.bn;
   {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)C_out};

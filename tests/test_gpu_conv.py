@@ -295,3 +295,21 @@ def test_auto_tiling_on_every_per_rank_conv_shape(n):
         err = float((y.float() - ref).norm() / ref.norm())
         assert torch.isfinite(y).all() and err < 2e-3, f"n={n} {ci}->{co} @{hw} s{stride}: rel-L2 {err:.3e}"
     _lib.device_status()
+
+
+@pytest.mark.parametrize("B,ci,co,H,W", [(2, 64, 64, 152, 8), (1, 128, 128, 16, 90), (1, 128, 512, 32, 68), (2, 64, 72, 6, 10)])
+@pytest.mark.parametrize("halo", [False, True])
+def test_strided_convolution_of_few_tiles(B, ci, co, H, W, halo):
+    """Stride 2 copies a tile's rows one at a time, sixteen of them at the narrowest widths, and splits K over CTAs where
+    there are few tiles."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    gen = torch.Generator().manual_seed(ci + co + W)
+    x, w = h16(torch.randn(B, ci, H, W, generator=gen)), h16(torch.randn(co, ci, 3, 3, generator=gen) / (9 * ci) ** 0.5)
+    b = h16(torch.randn(co, generator=gen))
+    rows = h16(torch.randn(2, B, ci, 1, W, generator=gen)) if halo else torch.zeros(2, B, ci, 1, W)
+    ref = torch.nn.functional.conv2d(torch.cat([rows[0], x, rows[1]], 2), w, b, stride=2, padding=(0, 1))[:, :, : H // 2]
+    top, bot = (nhwc(r).half().to(dev) if halo else None for r in rows)
+    y = _conv(ops, dev, x, w, b, 2, top, bot)
+    _lib.device_status()
+    assert_close(y, ref, what=f"strided conv {ci}->{co} {H}x{W}")
