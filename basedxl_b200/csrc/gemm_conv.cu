@@ -818,10 +818,12 @@ static std::atomic<int> g_clusters[64][5] = {};
 // `a_min_us` is a floor per k-block for the A operand path (the multi-row image copies of the convolution).  A
 // wider tile or a pair moves fewer bytes per FLOP; a narrower tile or a K split spreads the stream over more
 // SMs when there are few tiles; `heavy` epilogues read a residual or write fp32.  Of near equals the wider tile
-// is taken.  The choice is on average 0.6 % slower than the best configuration of each shape (at most 10 %); the
-// constants before, fitted while issuing a copy cost several times as much, chose 2.2 % and up to 41 %, on the
-// UNet's own layers up to 28 % (conv 2 x 640 x 64 x 64: 65.6 -> 51.1 us; GEMM 2048 x 2560 x 640: 16.3 -> 13.3 us;
-// 32768 x 2560 x 640: 105.8 -> 92.5 us).
+// is taken.  The constants before, fitted while issuing a copy cost several times as much, chose up to 28 % worse on
+// the UNet's own layers (conv 2 x 640 x 64 x 64: 65.6 -> 51.1 us; GEMM 2048 x 2560 x 640: 16.3 -> 13.3 us; 32768 x 2560 x
+// 640: 105.8 -> 92.5 us).  Swept again with the epilogues that the constants do not date from (residual rows and fp32
+// results in whole sectors, further accumulators of the fp32 product): over 120 shapes the choice is 2.0 % slower
+// than the best configuration in the mean (convolutions 0.7 %, fp32 products 1.0 %, linear layers 3.0 %), half of
+// them have the best, and the worst, 36 %, are products of two to four rows.
 static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int force_bn = 0, int force_split = 0,
                                int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0, int parts = 1, bool heavy = false) {
   const int sms = sm_count();
@@ -1381,7 +1383,7 @@ extern "C" int bxl_conv3x3_halo_f16(const void* x, long long x_img_stride, const
   const int K = 9 * C_in;
   const int tiles_x = (W_out + tw - 1) / tw, tiles_y = (H_out + th - 1) / th;
   const TileConfig tc = choose_tiles(B * tiles_x * tiles_y, C_out, K / kBK, false, g_force_bn, g_force_split,
-                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, conv_a_min_us(stride, th));
+                                     g_force_pair < 0 ? kDefaultPair : g_force_pair, conv_a_min_us(stride, th), 0, 1, residual != nullptr);
   const int BN = tc.bn;
   {
     uint64_t dims[2] = {(uint64_t)K, (uint64_t)C_out};
