@@ -29,7 +29,8 @@ def _req(cond: bool, msg: str) -> None:
 
 
 def _f16_cuda(t: torch.Tensor, name: str) -> None:
-    _req(t.is_cuda and t.dtype == torch.float16, f"{name}: expected a CUDA fp16 tensor, got {t.device} {t.dtype}")
+    if not (t.is_cuda and t.dtype == torch.float16):
+        raise ValueError(f"{name}: expected a CUDA fp16 tensor, got {t.device} {t.dtype}")
 
 
 # --------------------------------------------------------------------------- matmul
@@ -223,11 +224,12 @@ def gemm_ragged(a, b, bias=None, residual=None):
         _req(bias.shape == (N,) and bias.is_contiguous() and bias.device == a.device, "gemm_ragged: bad bias")
     out = torch.empty((M, N), device=a.device, dtype=torch.float16)
     # operands whose rows are not 16-byte aligned (or overlap) are copied by a launch of their own
-    copied = any(t.data_ptr() % 16 or ld % 8 or ld < t.shape[1] for t, ld in ((a, a.stride(0)), (b, N)))
+    lda = a.stride(0)
+    copied = lda % 8 or lda < K or N % 8 or (a.data_ptr() | b.data_ptr()) % 16
     l = _lib.lib()
     ws = torch.empty(max(l.bxl_gemm_ragged_workspace_bytes(M, N, K), 16), device=a.device, dtype=torch.uint8)
     _lib.check(
-        l.bxl_gemm_ragged_f16(_p(a), a.stride(0), _p(b), N, _p(bias), _p(residual), 0 if residual is None else residual.stride(0),
+        l.bxl_gemm_ragged_f16(_p(a), lda, _p(b), N, _p(bias), _p(residual), 0 if residual is None else residual.stride(0),
                               _p(out), N, M, N, K, _p(ws), ws.numel(), _stream()),
         l, kernels=2 if copied else 1,
     )
