@@ -70,6 +70,7 @@ struct alignas(64) GemmParams {
   // tiling chosen by the host
   int bn;                      // tile width: multiple of 32, 32..256
   int split;                   // K split over a cluster of `split` CTAs (1, 2 or 4)
+  int clusters;                // launched at most: what can be resident at one time (host side)
   int pair;                    // CTA pairs (cta_group::2): 256-row tiles, each CTA stages half of B (split == 1)
   int stages;                  // depth of the operand ring
   int b_static;                // B (weights) is not written by the preceding kernel: its copies start before the grid dependency wait
@@ -796,6 +797,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_conv_kernel(const __grid
 // ---------------------------------------------------------------------------------
 struct TileConfig {
   int bn, split, stages, pair;
+  int clusters;   // of the CTAs that share a tile: how many can be resident at one time
 };
 
 constexpr int kSmemLnExtra = 1024;           // the weight column-sum row of a GEMM with a folded LayerNorm
@@ -827,7 +829,7 @@ static std::atomic<int> g_clusters[64][5] = {};
 static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int force_bn = 0, int force_split = 0,
                                int force_pair = -1, double a_min_us = 0.0, int extra_smem = 0, int parts = 1, bool heavy = false) {
   const int sms = sm_count();
-  TileConfig best{128, 1, stages_for(128, 1, 0, extra_smem, parts), 0};
+  TileConfig best{128, 1, stages_for(128, 1, 0, extra_smem, parts), 0, sms};
   int at_once[5] = {0, sms, 0, 0, 0};
   for (int w = 2; w <= 4; w *= 2) at_once[w] = resident_clusters(gemm_conv_kernel<false, false, true, false>, kGemmThreads, kSmemBudget, w, g_clusters);
   double best_cost = 1e30;
@@ -858,7 +860,7 @@ static TileConfig choose_tiles(int tiles_m, int N, int num_kb, bool b_kn, int fo
         const double cost = (rounds * (kb_unit * kb_us + epi_us + pair_tile_us) + fill_us) * (1.0 - 0.05 * bn / 256.0);
         if (cost < best_cost - 1e-9) {
           best_cost = cost;
-          best = TileConfig{bn, split, st, pair};
+          best = TileConfig{bn, split, st, pair, clusters};
         }
       }
     }
@@ -881,7 +883,10 @@ static int launch_one(const GemmParams& p, int num_units, cudaStream_t stream) {
     configured[dev] = true;
   }
   const int width = kPair ? 2 : (kSplit ? p.split : 1);
-  int clusters = sm_count() / width;
+  // No more than the tile choice counted on: a cluster that has to wait for another one to end would start its whole
+  // share of the tiles only then.  33 clusters of 4 are resident, not 148 / 4 (forced splits of 4: 80 tiles of
+  // 1024 x 5120 x 1280 41.5 -> 30.3 us, 48 of 3000 x 5120 x 256 26.6 -> 22.8).
+  int clusters = p.clusters;
   if (clusters > num_units) clusters = num_units;
   if (clusters < 1) clusters = 1;
   return launch_kernel("gemm_conv_kernel launch", gemm_conv_kernel<kConv, kPair, kSplit, kTwo>, dim3(clusters * width), dim3(kGemmThreads), smem,
@@ -955,7 +960,7 @@ extern "C" int bxl_gemm_f16(const void* A, long long lda, const void* B, long lo
     if (int rc = encode_tmap_f16(&p.b_map[0], B, 2, dims, str, box)) return rc;
   }
   p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = b_is_kn ? 1 : 0;
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
   p.residual = static_cast<const __half*>(residual);
@@ -1064,7 +1069,7 @@ extern "C" int bxl_gemm_ragged_f16(const void* A, long long lda, const void* B, 
   }
   p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 1;
   // B is not static where the kernel above has just written it
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = (static_weights() && !b.dst) ? 1 : 0;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters, p.b_static = (static_weights() && !b.dst) ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
   p.residual = static_cast<const __half*>(residual);
@@ -1101,7 +1106,7 @@ extern "C" int bxl_gemm_dual_f16(const void* A, long long lda, const void* B, lo
     if (int rc = encode_tmap_f16(&p.b_map[0], B, 2, dims, str, box)) return rc;
   }
   p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 0;
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
   p.C = C1, p.ldc = ldc1, p.C2 = C2, p.ldc2 = ldc2, p.n_split = n1;
@@ -1135,7 +1140,7 @@ extern "C" int bxl_gemm_geglu_f16(const void* A, long long lda, const void* B, l
     if (int rc = encode_tmap_f16(&p.b_map[0], B, 2, dims, str, box)) return rc;
   }
   p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 0;
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(bias);
   p.C = C, p.ldc = ldc, p.out_f32 = 0, p.geglu = 1;
@@ -1198,7 +1203,7 @@ extern "C" int bxl_gemm_fused_f16(const bxl_gemm_fused_args* a, int* row_stats_p
     if (int rc = encode_tmap_f16(&p.b_map[0], a->B, 2, dims, str, box)) return rc;
   }
   p.M = M, p.N = N, p.K = K, p.parts = 1, p.b_kn = 0;
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters, p.b_static = static_weights() ? 1 : 0;
   p.n_fastest = linear_tile_order(M, N, K, tc.bn);
   p.bias = static_cast<const __half*>(a->bias);
   p.bias_f32 = a->bias_f32;
@@ -1308,7 +1313,7 @@ extern "C" int bxl_gemm_split_f32(const float* A, const float* B, float* C, int 
   }
   p.M = M, p.N = N, p.K = K, p.parts = 2, p.b_kn = 1;
   // b_static stays 0: the fp16 parts of B were written by the kernel launched just above
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters;
   p.C = C, p.ldc = N, p.out_f32 = 1;
   p.dev_status = st;
   return launch<false, true>(p, tiles_m, (N + BN - 1) / BN, s);
@@ -1392,7 +1397,7 @@ extern "C" int bxl_conv3x3_halo_f16(const void* x, long long x_img_stride, const
     if (int rc = encode_tmap_f16(&p.b_map[0], w_packed, 2, dims, str, box)) return rc;
   }
   p.M = B * H_out * W_out, p.N = C_out, p.K = K, p.parts = 1, p.b_kn = 0;
-  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.b_static = static_weights() ? 1 : 0;
+  p.bn = tc.bn, p.split = tc.split, p.stages = tc.stages, p.pair = tc.pair, p.clusters = tc.clusters, p.b_static = static_weights() ? 1 : 0;
   p.bias = static_cast<const __half*>(bias);
   p.bias_rows = static_cast<const __half*>(bias_rows);
   p.ld_bias_rows = bias_rows_stride > 0 ? bias_rows_stride : C_out;
