@@ -38,6 +38,7 @@ SIGNATURES = {
     "bxl_debug_force_tile_order": (_i, [_i]),
     "bxl_debug_force_attn_split": (_i, [_i]),
     "bxl_debug_force_attn_tiles": (_i, [_i, _i]),
+    "bxl_debug_exp2_f32": (_i, [_vp, _vp, _ll, _vp]),
     "bxl_gemm_f16": (_i, [_vp, _ll, _vp, _ll, _i, _vp, _vp, _ll, _vp, _ll, _i, _i, _i, _i, _vp]),
     "bxl_gemm_dual_f16": (_i, [_vp, _ll, _vp, _ll, _vp, _vp, _ll, _i, _vp, _ll, _i, _i, _i, _vp]),
     "bxl_gemm_geglu_f16": (_i, [_vp, _ll, _vp, _ll, _vp, _vp, _ll, _i, _i, _i, _vp]),

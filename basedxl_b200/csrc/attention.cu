@@ -910,6 +910,16 @@ __global__ void __launch_bounds__(kShortThreads, 512 / kShortKeys) attention_sho
   }
 }
 
+// Test hook: poly_exp2 by itself.
+__global__ void poly_exp2_kernel(const float* x, float* y, long long n) {
+  const long long i = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x);
+  if (i >= n) return;
+  float a, b;
+  unpair2(poly_exp2(pair2(x[i], i + 1 < n ? x[i + 1] : 0.f)), a, b);
+  y[i] = a;
+  if (i + 1 < n) y[i + 1] = b;
+}
+
 static int g_force_attn_split = 0, g_force_attn_groups = 0, g_force_attn_keys = 0;  // test hooks: 0 = choose
 
 // Tokens per key tile, query tiles per unit and K/V split: least rounds x time of a round.  Three groups of 64-token tiles
@@ -1001,6 +1011,12 @@ extern "C" int bxl_debug_force_attn_tiles(int groups, int keys) {
     return fail(kErrInvalidArg, "bxl_debug_force_attn_tiles: 0..3 query tiles (2 of 128 keys), 0, 64 or 128 keys");
   g_force_attn_groups = groups, g_force_attn_keys = keys;
   return kOk;
+}
+
+extern "C" int bxl_debug_exp2_f32(const float* x, float* y, long long n, void* stream) {
+  if (!x || !y || n <= 0) return fail(kErrInvalidArg, "bxl_debug_exp2_f32: bad argument");
+  poly_exp2_kernel<<<(unsigned)((n + 511) / 512), 256, 0, (cudaStream_t)stream>>>(x, y, n);
+  return check_cuda(cudaGetLastError(), "poly_exp2_kernel launch");
 }
 
 extern "C" int bxl_attn_fwd_f16(const void* q, long long q_img_stride, long long ld_q, const void* const* kv_slots,

@@ -73,6 +73,10 @@ int bxl_debug_force_attn_split(int split);
  * forced plan (K/V split included) does not fit returns an error.  No counterpart in the reference. */
 int bxl_debug_force_attn_tiles(int groups, int keys);
 
+/* Test hook: y[i] = 2^x[i] by the polynomial that the attention kernel takes for part of its exponentials.  No
+ * counterpart in the reference. */
+int bxl_debug_exp2_f32(const float* x, float* y, long long n, void* stream);
+
 /* ---- matmul ------------------------------------------------------------- */
 
 /* C[M,N] = A[M,K] * B (+ bias[N]) (+ residual[M,N]); fp16 operands, fp32

@@ -307,3 +307,23 @@ def test_attention_with_few_keys(keys, Lq, offset):
     _lib.device_status()
     assert_close(out, po._sdpa_heads(q, kv, heads), what=f"attention of {keys} keys, Lq {Lq}")
     assert bool((store[..., :offset] == 7).all()) and bool((store[..., offset + C :] == 7).all())
+
+
+def test_exponential_on_the_fma_pipe():
+    """2^x by the polynomial: a relative error of at most 2.5e-7 (the bound of the special-function unit is 2^-22 =
+    2.4e-7) wherever the result counts (x <= 8), as good as zero below -120, exactly one at zero, NaN, an odd count."""
+    dev = cuda_or_skip()
+    _lib, ops = _ops()
+    x = torch.cat([torch.linspace(-30, 12, 200001), torch.arange(-110, 120).float(), torch.tensor([0.0, 0.5, -0.5, 126.4, -119.9])])
+    limits = torch.tensor([-120.0, -200.0, -1e30, float("-inf"), float("nan")])
+    xd = torch.cat([x, limits]).to(dev)
+    assert xd.numel() % 2 == 1
+    y = torch.full_like(xd, 7.0)
+    l = _lib.lib()
+    _lib.check(l.bxl_debug_exp2_f32(xd.data_ptr(), y.data_ptr(), xd.numel(), torch.cuda.current_stream().cuda_stream), l, kernels=0)
+    y = y.cpu()
+    ref = torch.exp2(x.double())
+    assert float(((y[: x.numel()].double() - ref).abs() / ref).max()) <= 2.5e-7
+    assert float(y[(x == 0).nonzero()[0, 0]]) == 1.0
+    t = y[x.numel() :]
+    assert bool((t[:4] >= 0).all()) and bool((t[:4] < 1e-35).all()) and bool(torch.isnan(t[4]))
