@@ -130,7 +130,8 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 // softmax's narrowest unit.  x = n + f with n the nearest integer (the sum with 1.5 * 2^23 + 127 leaves n + 127 in
 // the low mantissa bits), 2^f by a degree-5 polynomial fitted to |f| <= 0.5 for the smallest relative error
 // (2.1e-7 in fp32 arithmetic, the error bound of the special-function unit), times 2^n built from those bits.
-// x <= 8 here; below -120 the result is as good as zero; NaN stays NaN.
+// x <= 8, unless the caller's scale is negative: the result is then wrong from 128 on, where fp16 has long overflowed in
+// the other scores; below -120 it is as good as zero; NaN stays NaN.
 __device__ __forceinline__ f32x2 poly_exp2(f32x2 x) {
   float x0, x1;
   unpair2(x, x0, x1);
